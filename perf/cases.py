@@ -2,7 +2,8 @@
 
 A case is a dict of plain values.  ``listed()`` gives the fixed ones, ``draw(rng)`` one more of the same ranges,
 ``prepare`` what a program holds before the call (a session or an engine with its weights, and the inputs),
-``run`` one pass through the public entry points, ``work`` the bytes and operations a pass cannot do without.
+``run`` one pass through the public entry points, ``exact`` what a session's pass gives in 64 bits, ``work`` the bytes
+and operations a pass cannot do without.
 
 Models are the ones the package builds itself, with random weights.  Two scales differ from the builders' defaults,
 both in the serving cases: token embeddings are as large as in a trained decoder (standard deviation 0.14 for GPT-2,
@@ -16,6 +17,7 @@ import functools
 import math
 
 import torch
+import torch.nn.functional as F
 
 from ronn_b200 import Model, SessionOptions
 from ronn_b200.models.bitnet_llama import BitNetConfig, build_bitnet_llama
@@ -206,6 +208,13 @@ def prepare(case, seed):
     if model.endswith("-serve"):
         return _prepare_serving(case, seed)
     session = _session(model, case.get("image", 0), case["dtype"], case.get("graph", False))
+    feed = _feed(case, seed)
+    session.run(feed)                            # kernels loaded, and with graph replay the graph of this shape captured
+    return dict(case=case, session=session, feed=feed)
+
+
+def _feed(case, seed):
+    model = case["model"]
     gen = torch.Generator(device="cuda").manual_seed(seed)
     if model == "mlp784":
         feed = {"input": torch.rand(case["batch"], 784, generator=torch.Generator().manual_seed(seed))}
@@ -221,8 +230,7 @@ def prepare(case, seed):
             if case["padded"]:
                 lens = torch.randint(max(1, case["seq"] // 4), case["seq"] + 1, lens.shape, generator=gen, device="cuda")
             feed["attention_mask"] = (torch.arange(case["seq"], device="cuda")[None, :] < lens).to(torch.int64)
-    session.run(feed)                            # kernels loaded, and with graph replay the graph of this shape captured
-    return dict(case=case, session=session, feed=feed)
+    return feed
 
 
 def run(state):
@@ -232,6 +240,103 @@ def run(state):
     tokens = engine.generate(state["prompts"], state["params"])
     # the tokens, and the keys and values that the engine holds after the pass
     return dict(tokens=torch.tensor(tokens, dtype=torch.int32), keys=engine.runner.kcache, values=engine.runner.vcache)
+
+
+# ---------------------------------------------------------------------------------------------------- the same in 64 bits
+@functools.lru_cache(maxsize=2)
+def _weights64(model, image, dtype):
+    """The weights a session starts from, in 64 bits on the device."""
+    t = _DTYPES[dtype]
+    if model == "mlp784":
+        g = build_mlp784(seed=1)
+    elif model == "resnet18":
+        g = build_resnet18(dtype=t, seed=1, image=image)
+    elif model == "distilbert":
+        g = build_distilbert(DistilBertConfig.base(), dtype=t, seed=1)
+    else:
+        g = build_gpt2(GPT2Config.small(), dtype=t, seed=1)
+    return {k: v.cuda().double() for k, v in g.initializers.items() if v.is_floating_point()}
+
+
+def _resnet64(w, x):
+    def conv(x, n, stride, pad, eps=1e-5):
+        y = F.conv2d(x, w[n + ".weight"], stride=stride, padding=pad)
+        return F.batch_norm(y, w[n + ".bn.running_mean"], w[n + ".bn.running_var"], w[n + ".bn.weight"], w[n + ".bn.bias"], eps=eps)
+
+    x = F.max_pool2d(conv(x, "stem", 2, 3).relu(), 3, 2, 1)
+    for stage in range(4):
+        for blk in range(2):
+            n, stride = f"layer{stage + 1}.{blk}", 2 if stage > 0 and blk == 0 else 1
+            y = conv(conv(x, n + ".a", stride, 1).relu(), n + ".b", 1, 1)
+            skip = conv(x, n + ".down", stride, 0) if n + ".down.weight" in w else x
+            x = (y + skip).relu()
+    return x.mean((2, 3)) @ w["fc.weight"].t() + w["fc.bias"]
+
+
+def _attend64(q, k, v, heads, mask):
+    b, s, h = q.shape
+    q, k, v = (t.view(b, s, heads, h // heads).transpose(1, 2) for t in (q, k, v))
+    p = (q @ k.transpose(-1, -2) / math.sqrt(h // heads)).masked_fill(~mask, float("-inf")).softmax(-1)
+    return (p @ v).transpose(1, 2).reshape(b, s, h)
+
+
+def _distilbert64(w, c, ids, mask):
+    def lin(x, n):
+        return x @ w[n + ".weight"] + w[n + ".bias"]
+
+    def norm(x, n):
+        return F.layer_norm(x, (c.dim,), w[n + ".weight"], w[n + ".bias"], c.eps)
+
+    x = w["embeddings.word_embeddings.weight"][ids] + w["embeddings.position_embeddings.weight"][:ids.shape[1]]
+    x = norm(x, "embeddings.LayerNorm")
+    for i in range(c.n_layers):
+        p = f"transformer.layer.{i}"
+        q, k, v = (lin(x, f"{p}.attention.{n}_lin") for n in "qkv")
+        x = norm(lin(_attend64(q, k, v, c.n_heads, mask[:, None, None, :] > 0), p + ".attention.out_lin") + x, p + ".sa_layer_norm")
+        f = lin(F.gelu(lin(x, p + ".ffn.lin1"), approximate="tanh"), p + ".ffn.lin2")
+        x = norm(f + x, p + ".output_layer_norm")
+    return x
+
+
+def _gpt2_64(w, c, ids):
+    def lin(x, n):
+        return x @ w[n + ".weight"] + w[n + ".bias"]
+
+    def norm(x, n):
+        return F.layer_norm(x, (c.n_embd,), w[n + ".weight"], w[n + ".bias"], c.layer_norm_epsilon)
+
+    s = ids.shape[1]
+    seen = torch.ones(s, s, dtype=torch.bool, device=ids.device).tril()
+    x = w["wte"][ids] + w["wpe"][:s]
+    for i in range(c.n_layer):
+        p = f"h.{i}"
+        q, k, v = lin(norm(x, p + ".ln_1"), p + ".attn.c_attn").chunk(3, -1)
+        x = x + lin(_attend64(q, k, v, c.n_head, seen), p + ".attn.c_proj")
+        x = x + lin(F.gelu(lin(norm(x, p + ".ln_2"), p + ".mlp.c_fc"), approximate="tanh"), p + ".mlp.c_proj")
+    return norm(x, "ln_f")
+
+
+def exact(case, seed):
+    """Sessions in 64 bits, with the weights they start from.  An engine chooses tokens and then reads its own choices:
+    its pass has no such value."""
+    model = case["model"]
+    if model.endswith("-serve"):
+        return None
+    feed = _feed(case, seed)
+    w = _weights64(model, case.get("image", 0), case["dtype"])
+    with torch.no_grad():
+        if model == "mlp784":
+            x = feed["input"].cuda().double()
+            x = (x @ w["fc1.weight"] + w["fc1.bias"]).relu()
+            return {"probs": (x @ w["fc2.weight"] + w["fc2.bias"]).softmax(-1)}
+        if model == "resnet18":
+            return {"logits": torch.cat([_resnet64(w, x.double()) for x in feed["input"].split(8)])}
+        if model == "distilbert":
+            c, mask = DistilBertConfig.base(), feed["attention_mask"]
+            parts = [_distilbert64(w, c, i, m) for i, m in zip(feed["input_ids"].split(16), mask.split(16))]
+            return {"last_hidden_state": torch.cat(parts)}
+        hidden = torch.cat([_gpt2_64(w, GPT2Config.small(), i) for i in feed["input_ids"].split(4)])
+        return {"last_hidden_state": hidden, "logits": hidden @ w["wte"].t()}
 
 
 # ---------------------------------------------------------------------------------------------------- what a pass needs
