@@ -106,6 +106,7 @@ int pick_bn(int M, int N) {
 // Pipeline depth.  A CTA that is alone on its SM is fed by the bytes it keeps in flight, so when the whole problem
 // is at most one CTA per SM the ring is twice as deep (6 / 8 / 10 stages for BN 128 / 64 / 32, one CTA per SM)
 // instead of two co-resident CTAs with half the ring each.  bn | 0x1000 forces the deep ring, bn | 0x2000 the shallow.
+bool skinny_rule(int M, int N, int K);       // gemm_skinny.cu
 static int deep_mode(int bn) { return (bn & 0x1000) ? 1 : ((bn & 0x2000) ? 0 : -1); }
 static int wants_deep(int M, int N, int bn, int splitk) {
   static int forced = -2;                                  // RONN_GEMM_RING = deep | shallow overrides the choice
@@ -122,6 +123,10 @@ static int wants_deep(int M, int N, int bn, int splitk) {
 
 using namespace ronn;
 
+extern "C" int ronn_gemm_skinny(const void* A, const void* W, void* C, const void* bias, const void* residual,
+                                const void* gamma, const void* beta, float eps, int norm, int M, int N, int K, long lda,
+                                long ldw, long ldc, int dtype, int act, int out_fp32, cudaStream_t stream);
+
 // dtype: 0 = bf16, 1 = fp16.  act: 0 none, 1 relu, 2 gelu.  bn: 0 = auto, else 32|64|128|256 (| 0x1000 deep ring,
 // | 0x2000 shallow ring; default picks by tile count).
 // lda/ldw/ldc in elements; K and the leading dimensions must be multiples of 8.
@@ -131,6 +136,8 @@ extern "C" int ronn_gemm(const void* A, const void* W, void* C, const void* bias
                          uint32_t* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   if ((K & 7) || (lda & 7) || (ldw & 7)) return -2;
+  if (bn == 0 && skinny_rule(M, N, K))
+    return ronn_gemm_skinny(A, W, C, bias, residual, nullptr, nullptr, 0.f, 0, M, N, K, lda, ldw, ldc, dtype, act, out_fp32, stream);
   int deep = deep_mode(bn);
   bn &= 0xfff;
   if (bn == 0) bn = pick_bn(M, N);

@@ -92,6 +92,38 @@ def gemm(a: torch.Tensor, w_nk: torch.Tensor, bias: Optional[torch.Tensor] = Non
     return out
 
 
+def norm_gemm_ok(rows: int, k: int) -> bool:
+    """Sizes ``norm_gemm`` takes: few rows, a row short enough to stay in the registers of one CTA."""
+    return 0 < rows <= 8 and k <= 1024 and k % 8 == 0
+
+
+def skinny_down_ok(rows: int, n: int, k: int) -> bool:
+    """Whether a long-K projection is faster as one skinny GEMM followed by a norm kernel than as split-K partial sums
+    whose reduction applies the norm (measured, us with the norm: N 1024 K 4096: 16 rows 8.4 / 9.9, 32 rows 9.2 / 10.1,
+    48 rows 13.0 / 10.3; N 768 K 3072: 48 rows 8.1 / 9.7, 64 rows 10.9 / 10.0): up to 8 Mi values of weights x passes."""
+    return -(-rows // 16) * n * k <= 8 << 20
+
+
+def norm_gemm(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor], eps: float, norm: str,
+              w_nk: torch.Tensor, bias: Optional[torch.Tensor] = None, activation: str = "",
+              out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """act(norm(x) @ w_nk^T + bias) for few rows (``norm_gemm_ok``) in one launch; norm: "layernorm" | "rmsnorm"."""
+    M, K = x.shape
+    N = w_nk.shape[0]
+    if not norm_gemm_ok(M, K) or w_nk.shape[1] != K or x.stride(1) != 1 or w_nk.stride(1) != 1:
+        raise KernelError(f"norm_gemm does not take x {tuple(x.shape)} w {tuple(w_nk.shape)}")
+    if x.dtype not in (torch.bfloat16, torch.float16) or any(t is not None and t.dtype != x.dtype for t in (w_nk, gamma, beta, bias)):
+        raise KernelError("norm_gemm needs bf16/fp16 operands of one dtype")
+    if out is None:
+        out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+    rc = _native.cuda().ronn_gemm_skinny(x.data_ptr(), w_nk.data_ptr(), out.data_ptr(), _ptr(bias), None, gamma.data_ptr(),
+                                         _ptr(beta), float(eps), {"layernorm": 1, "rmsnorm": 2}[norm], M, N, K, x.stride(0),
+                                         w_nk.stride(0), out.stride(0), _DT[x.dtype], _ACT[activation],
+                                         1 if out.dtype == torch.float32 else 0, _stream())
+    _check(rc, "norm_gemm")
+    return out
+
+
 def _norm(x, gamma, beta, residual, eps, rms, sum_out):
     H = x.shape[-1]
     x2 = x.reshape(-1, H)

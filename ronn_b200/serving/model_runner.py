@@ -107,6 +107,8 @@ class DecoderRunner:
         self.tp, self.rank = self.comm.world, self.comm.rank
         self.dtype = {"bf16": torch.bfloat16, "fp16": torch.float16, "fp32": torch.float32}[cfg.dtype]
         self.ops = make_ops(cfg.backend, device)
+        from ..ops.kernels import norm_gemm_ok, skinny_down_ok
+        self._norm_gemm_ok, self._skinny_down_ok = norm_gemm_ok, skinny_down_ok
         if cfg.backend == "kernels" and self.dtype == torch.float32:
             raise SessionError("the kernel backend computes in bf16 or fp16")
         a = arch
@@ -269,6 +271,10 @@ class DecoderRunner:
         max_ctx = self.step_ctx if (ops.name == "torch" and self.step_ctx) else self.cfg.max_model_len
         split_down = (ops.name == "kernels" and self.tp == 1 and x.shape[0] <= 512 and not a.bitlinear
                       and self.layers[0]["down"].w is not None and self.layers[0]["down"].w.shape[1] >= 2048)
+        # few rows, one rank: the norm joins the projection that reads it, and the down projection is one launch
+        fuse_norm = (ops.name == "kernels" and self.tp == 1 and not a.bitlinear and self._norm_gemm_ok(x.shape[0], a.hidden))
+        if split_down and self._skinny_down_ok(x.shape[0], *self.layers[0]["down"].w.shape):
+            split_down = False
         # one rank, prefill-sized batches: the projections that end a half block run as a cluster GEMM whose epilogue
         # also applies the next norm.  Not for decode: with one or two row tiles only 8-16 CTAs would stream the whole
         # weight matrix (measured 2x slower than split-K + finalize there).
@@ -300,6 +306,8 @@ class DecoderRunner:
         for li, L in enumerate(self.layers):
             if h_next is None and L["qkv"].packed is not None:
                 qkv = self._norm_linear(x, L["ln1"], L["qkv"])
+            elif h_next is None and fuse_norm:
+                qkv = ops.norm_gemm(x, L["ln1"], a.norm, a.eps, L["qkv"].w, L["qkv"].bias)
             else:
                 h = h_next if h_next is not None else self._norm(x, L["ln1"])
                 qkv = self._linear(h, L["qkv"])
@@ -334,6 +342,10 @@ class DecoderRunner:
                     f = QuantAct(*KB.swiglu_quant_int8(gu), gu.dtype)
                 else:
                     f = ops.swiglu_fused(gu)
+            elif h is None and fuse_norm:
+                f = ops.norm_gemm(x, L["ln2"], a.norm, a.eps, L["up"].w, L["up"].bias, "gelu" if a.mlp == "gelu" else "")
+                if a.mlp != "gelu":
+                    f = ops.swiglu_fused(f)
             else:
                 if h is None:
                     h = self._norm(x, L["ln2"])
@@ -344,13 +356,18 @@ class DecoderRunner:
             nxt = self.layers[li + 1]["ln1"] if li + 1 < len(self.layers) else (self.lnf if decode else None)
             x, h_next = row_parallel(f, L["down"], x, nxt, True,
                                      quant_next=li + 1 < len(self.layers) and self.layers[li + 1]["qkv"].packed is not None)
+        logits = None
         if h_next is not None:
             x = h_next                                   # final norm already applied by the last reduction pass
         else:
             if not decode:
                 x = ops.gather_rows(x, b["sample_index_clamped"])
-            x = self._norm(x, self.lnf)
-        logits = ops.lm_head(x, self.lm_head)
+            if ops.name == "kernels" and self.tp == 1 and self._norm_gemm_ok(x.shape[0], a.hidden):
+                logits = ops.norm_gemm(x, self.lnf, a.norm, a.eps, self.lm_head, logits=True)
+            else:
+                x = self._norm(x, self.lnf)
+        if logits is None:
+            logits = ops.lm_head(x, self.lm_head)
         if want_logits:
             return logits if self.tp == 1 else self.gather_vocab(logits, comm)
         if self.tp == 1:

@@ -127,9 +127,16 @@ class KernelOps:
         """fp32 logits [rows, vocab].  The buffer's row stride is padded to a multiple of 8 values: with an odd
         vocabulary (50257) as the stride every row would start off a 16-byte boundary and the GEMM epilogue would fall
         back to scalar stores (measured: 113 us instead of about 30 for 256 x 50257 x 1024)."""
+        return self.K.gemm(x, w_nk, out=self._logits(x, w_nk), out_fp32=True)
+
+    def _logits(self, x, w_nk):
         n = w_nk.shape[0]
-        buf = torch.empty((x.shape[0], -(-n // 8) * 8), dtype=torch.float32, device=x.device)
-        return self.K.gemm(x, w_nk, out=buf[:, :n], out_fp32=True)
+        return torch.empty((x.shape[0], -(-n // 8) * 8), dtype=torch.float32, device=x.device)[:, :n]
+
+    def norm_gemm(self, x, norm_p, norm_kind, eps, w_nk, bias=None, activation="", logits=False):
+        """norm(x) and the projection that reads it in one launch (few rows: ``ops.kernels.norm_gemm_ok``)."""
+        return self.K.norm_gemm(x, norm_p[0], norm_p[1] if len(norm_p) > 1 else None, eps, norm_kind, w_nk, bias, activation,
+                                out=self._logits(x, w_nk) if logits else None)
 
     def layernorm(self, x, w, b, eps):
         return self.K.layernorm(x, w, b, eps)
