@@ -25,10 +25,12 @@ struct DenseEpilogue {
     // re-shaping the stores through shared memory pays for bandwidth-bound results; a decode-sized GEMM (a few row
     // tiles) is a latency chain and keeps the direct stores
     const bool staged = stage != nullptr && M >= 1024 && !out_fp32 && (gn + 32 <= N) && ((ldc & 7) == 0);
-    if (gm >= M && !staged) return;
-    if (gm >= M) {                               // staged path: rows past the end only take part in the exchange
+    const bool ragged = stage != nullptr && !out_fp32 && (ldc & 7) != 0;
+    if (gm >= M && !staged && !ragged) return;
+    if (gm >= M) {                               // staged paths: rows past the end only take part in the exchange
       __syncwarp();
-      store_staged<T>(stage, gm - (threadIdx.x & 31), gn);
+      if (staged) store_staged<T>(stage, gm - (threadIdx.x & 31), gn);
+      else store_ragged<T>(stage, gm - (threadIdx.x & 31), gn);
       return;
     }
     float v[32];
@@ -93,7 +95,7 @@ struct DenseEpilogue {
         for (int i = 0; i < 32; ++i)
           if (gn + i < N) out[i] = v[i];
       }
-    } else if (staged) {
+    } else if (staged || ragged) {
       uint8_t* mine = stage + (threadIdx.x & 31) * 80;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -103,7 +105,8 @@ struct DenseEpilogue {
         *reinterpret_cast<Vec8*>(mine + j * 16) = pack8<T>(f);
       }
       __syncwarp();
-      store_staged<T>(stage, gm - (threadIdx.x & 31), gn);
+      if (staged) store_staged<T>(stage, gm - (threadIdx.x & 31), gn);
+      else store_ragged<T>(stage, gm - (threadIdx.x & 31), gn);
     } else {
       T* out = reinterpret_cast<T*>(C) + size_t(gm) * ldc + gn;
       if (full) {
@@ -136,6 +139,21 @@ struct DenseEpilogue {
       }
     }
     __syncwarp();                                // the stage is free for the warp's next chunk
+  }
+
+  // The same for rows that do not start on 16-byte boundaries (ldc not a multiple of 8): lane l writes column gn + l,
+  // so a store instruction covers one run of 64 bytes of one row.  Stored from the accumulator layout (lane = row) each
+  // instruction touched 32 rows, two bytes in each.
+  template <class T>
+  __device__ __forceinline__ void store_ragged(const uint8_t* stage, int base_row, int gn) const {
+    const int lane = threadIdx.x & 31;
+    const int rows = min(32, M - base_row);
+    if (gn + lane < N) {
+      T* dst = reinterpret_cast<T*>(C) + size_t(base_row) * ldc + gn + lane;
+#pragma unroll 8
+      for (int i = 0; i < rows; ++i) dst[size_t(i) * ldc] = *reinterpret_cast<const T*>(stage + i * 80 + lane * 2);
+    }
+    __syncwarp();
   }
 };
 

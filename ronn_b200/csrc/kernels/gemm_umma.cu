@@ -142,6 +142,8 @@ extern "C" int ronn_gemm(const void* A, const void* W, void* C, const void* bias
   bn &= 0xfff;
   if (bn == 0) bn = pick_bn(M, N);
   if (deep < 0) deep = wants_deep(M, N, bn, 1);
+  // rows off the 16-byte grid leave through the store-staging area, which only the deep rings carry
+  if (!out_fp32 && (ldc & 7)) deep = 1;
   CUtensorMap ma, mb;
   int rc = make_tmap_2d(&ma, A, uint64_t(M), uint64_t(K), uint64_t(lda), PG_BM, 64, 2);
   if (rc) return rc - 20;

@@ -1,0 +1,29 @@
+"""Tile shapes and store paths of the tcgen05 GEMM against a 64-bit product of the same rounded operands: one rounding of the
+result to 16 bits (half a unit in the last place, so below 2^-8 for bf16 and 2^-11 for fp16 as a relative error of the
+whole)."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+TOL = {torch.bfloat16: 2 ** -8, torch.float16: 2 ** -11}
+
+
+def _operands(M, N, Kd, dtype):
+    g = torch.Generator(device="cuda").manual_seed(M * 131 + N + Kd)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").to(dtype)
+    return r(M, Kd), (r(N, Kd).float() / Kd ** 0.5).to(dtype), r(N), r(M, N)
+
+
+# output rows that do not start on 16-byte boundaries: rows past the end of the last tile, column tiles cut short, every
+# tile width the automatic choice takes there
+@pytest.mark.parametrize("M,N,Kd", [(129, 1001, 64), (300, 131, 72), (1030, 4099, 128), (2600, 8009, 64), (513, 7, 8)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_rows_off_the_16_byte_grid(M, N, Kd, dtype):
+    from ronn_b200.ops import kernels as K
+    x, w, bias, res = _operands(M, N, Kd, dtype)
+    out = torch.full((M + 1, N), 7.0, dtype=dtype, device="cuda")
+    K.gemm(x, w, bias, res, "relu", out=out[:M])
+    K.check_status()
+    ref = F.relu(x.double() @ w.double().t() + bias.double()) + res.double()
+    assert ((out[:M].double() - ref).norm() / ref.norm()).item() < TOL[dtype] and bool((out[M] == 7).all())
