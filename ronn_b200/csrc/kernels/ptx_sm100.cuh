@@ -134,6 +134,17 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+// Im2col load of an NHWC tensor, no multicast: channels c.. of the filter tap at (off_w, off_h) for consecutive output
+// positions starting with the window whose top-left corner is (w, h) of image n.  c * 2 must be a multiple of 16 bytes.
+__device__ __forceinline__ void tma_load_im2col(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int32_t c, int32_t w,
+                                                int32_t h, int32_t n, uint16_t off_w, uint16_t off_h) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], "
+      "{%7, %8};" ::"r"(smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h)
+      : "memory");
+}
+
 // ------------------------------------------------------------------------- TMEM
 // Executed by one full warp.  ncols: power of two in [32, 512].  The base address lands in *smem_result.
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {
@@ -158,6 +169,17 @@ __device__ __forceinline__ uint64_t umma_desc_k128(uint32_t smem_addr) {
   d |= uint64_t(1024 >> 4) << 32;                // stride byte offset: 8 rows * 128 B
   d |= uint64_t(1) << 46;                        // descriptor version (Blackwell)
   d |= uint64_t(2) << 61;                        // layout: SWIZZLE_128B
+  return d;
+}
+
+// The same for rows of 32 bytes with the 32-byte swizzle (one K = 16 step of 16-bit values): 8-row groups of 256 bytes.
+__device__ __forceinline__ uint64_t umma_desc_k32(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= uint64_t((smem_addr & 0x3FFFF) >> 4);
+  d |= uint64_t(1) << 16;
+  d |= uint64_t(256 >> 4) << 32;
+  d |= uint64_t(1) << 46;
+  d |= uint64_t(6) << 61;                        // layout: SWIZZLE_32B
   return d;
 }
 

@@ -23,11 +23,18 @@
 //   static constexpr bool kForceStage                                 true: `stage` below is never null
 //   void epilogue(int t, int m0, int n0, int row, int col, uint32_t (&acc)[32], uint8_t* stage)   row/col within the
 //        tile; stage: 32 x 80 bytes of shared memory owned by the calling warp (to re-shape its stores), or null
+//   static constexpr bool kTapA (optional)                            true: the A half of an atom is four tiles of 128 rows
+//        x 32 bytes (32-byte swizzle), one per K = 16 step, instead of one tile of 128 rows x 128 bytes
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 #include "ptx_sm100.cuh"
 
 namespace ronn {
+
+template <class P, class = void> struct TapA : std::false_type {};
+template <class P> struct TapA<P, std::void_t<decltype(P::kTapA)>> : std::bool_constant<P::kTapA> {};
 
 constexpr int PG_BM = 128;
 constexpr int PG_EPI_WARPS = 8;                  // two warps per TMEM lane quarter, each drains half of the columns
@@ -164,13 +171,14 @@ __device__ __forceinline__ void gemm_persistent(uint8_t* dyn_smem, Problem& prob
 #pragma unroll
           for (int a = 0; a < KA; ++a) {
             if (a < na) {
-              const uint64_t adesc = umma_desc_k128(sa + a * L::ATOM_BYTES);
+              constexpr uint64_t ASTEP = TapA<Problem>::value ? (PG_BM * 32) >> 4 : 2;      // 16-byte units per K = 16 step
+              const uint64_t adesc = TapA<Problem>::value ? umma_desc_k32(sa + a * L::ATOM_BYTES) : umma_desc_k128(sa + a * L::ATOM_BYTES);
               const uint64_t bdesc = umma_desc_k128(sa + a * L::ATOM_BYTES + L::A_BYTES);
 #pragma unroll
               for (int k = 0; k < 4; ++k) {      // 4 x 32 bytes of K per 128-byte row
                 const uint32_t acc = (sb | a | k) != 0;
-                if (KIND == 0) umma_f16(tmem_d, adesc + 2 * k, bdesc + 2 * k, idesc, acc);
-                else umma_i8(tmem_d, adesc + 2 * k, bdesc + 2 * k, idesc, acc);
+                if (KIND == 0) umma_f16(tmem_d, adesc + ASTEP * k, bdesc + 2 * k, idesc, acc);
+                else umma_i8(tmem_d, adesc + ASTEP * k, bdesc + 2 * k, idesc, acc);
               }
             }
           }
@@ -217,26 +225,23 @@ __device__ __forceinline__ void gemm_persistent(uint8_t* dyn_smem, Problem& prob
         const int c0 = half * HALF;
         uint32_t r0[32], r1[32];
         tmem_ld_32x32(tacc + uint32_t(c0), r0);
-        if (HALF == 32) {
-          tmem_ld_wait();
+        auto release = [&]() {                   // the last load of this buffer has landed
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&acc_empty[buf]);
-          prob.epilogue(t, m0, n0, row, c0, r0, stage_w);
-        } else {
+        };
+        constexpr int NC = HALF / 32;            // 32-column pieces: 1, 2, 3 or 4
 #pragma unroll 1
-          for (int col = c0; col < c0 + HALF; col += 64) {
+        for (int c = 0; c < NC; c += 2) {
+          const int col = c0 + c * 32;
+          tmem_ld_wait();
+          if (c + 1 < NC) tmem_ld_32x32(tacc + uint32_t(col + 32), r1);
+          else release();
+          prob.epilogue(t, m0, n0, row, col, r0, stage_w);
+          if (c + 1 < NC) {
             tmem_ld_wait();
-            tmem_ld_32x32(tacc + uint32_t(col + 32), r1);
-            prob.epilogue(t, m0, n0, row, col, r0, stage_w);
-            tmem_ld_wait();
-            if (col + 64 < c0 + HALF) {
-              tmem_ld_32x32(tacc + uint32_t(col + 64), r0);
-            } else {
-              tc_fence_before_sync();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&acc_empty[buf]);
-            }
+            if (c + 2 < NC) tmem_ld_32x32(tacc + uint32_t(col + 64), r0);
+            else release();
             prob.epilogue(t, m0, n0, row, col + 32, r1, stage_w);
           }
         }
