@@ -37,29 +37,46 @@ struct DenseEpilogue {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
     const bool full = (gn + 32 <= N) && ((ldc & 7) == 0);
-    if (bias) {
-      const T* b = reinterpret_cast<const T*>(bias) + gn;
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (full || gn + i < N) v[i] += Cvt<T>::to_f(b[i]);
-    }
-    if (residual && res_first) {
+    // the residual row is fetched first: its latency passes under the bias and the activation
+    Vec8 rp[4];
+    if (residual && full) {
       const T* res = reinterpret_cast<const T*>(residual) + size_t(gm) * ldc + gn;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) rp[j] = *reinterpret_cast<const Vec8*>(res + j * 8);
+    }
+    auto add_residual = [&]() {
       if (full) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          Vec8 pk = *reinterpret_cast<const Vec8*>(res + j * 8);
           float f[8];
-          unpack8<T>(pk, f);
+          unpack8<T>(rp[j], f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[j * 8 + i] += f[i];
+        }
+      } else {
+        const T* res = reinterpret_cast<const T*>(residual) + size_t(gm) * ldc + gn;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (gn + i < N) v[i] += Cvt<T>::to_f(res[i]);
+      }
+    };
+    if (bias) {
+      const T* b = reinterpret_cast<const T*>(bias) + gn;
+      if (gn + 32 <= N && (reinterpret_cast<uintptr_t>(b) & 15) == 0) {      // four 16-byte loads instead of 32 of two bytes
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float f[8];
+          unpack8<T>(*reinterpret_cast<const Vec8*>(b + j * 8), f);
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[j * 8 + i] += f[i];
         }
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i)
-          if (gn + i < N) v[i] += Cvt<T>::to_f(res[i]);
+          if (gn + i < N) v[i] += Cvt<T>::to_f(b[i]);
       }
     }
+    if (residual && res_first) add_residual();
     if (act == 1) {
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i], 0.f);
@@ -67,23 +84,7 @@ struct DenseEpilogue {
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = gelu_tanh_f(v[i]);
     }
-    if (residual && !res_first) {
-      const T* res = reinterpret_cast<const T*>(residual) + size_t(gm) * ldc + gn;
-      if (full) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          Vec8 pk = *reinterpret_cast<const Vec8*>(res + j * 8);
-          float f[8];
-          unpack8<T>(pk, f);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[j * 8 + i] += f[i];
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (gn + i < N) v[i] += Cvt<T>::to_f(res[i]);
-      }
-    }
+    if (residual && !res_first) add_residual();
     if (out_fp32) {
       float* out = reinterpret_cast<float*>(C) + size_t(gm) * ldc + gn;
       if (full && (ldc & 3) == 0) {

@@ -27,3 +27,17 @@ def test_rows_off_the_16_byte_grid(M, N, Kd, dtype):
     K.check_status()
     ref = F.relu(x.double() @ w.double().t() + bias.double()) + res.double()
     assert ((out[:M].double() - ref).norm() / ref.norm()).item() < TOL[dtype] and bool((out[M] == 7).all())
+
+
+# bias on and off the 16-byte grid, columns cut short, residual rows with and without whole pieces
+@pytest.mark.parametrize("M,N,Kd", [(200, 264, 64), (1100, 1000, 128), (1100, 260, 64)])
+@pytest.mark.parametrize("off", [0, 1, 8])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_bias_and_residual_alignment(M, N, Kd, off, dtype):
+    from ronn_b200.ops import kernels as K
+    x, w, _, res = _operands(M, N, Kd, dtype)
+    bias = torch.randn(N + off, device="cuda").to(dtype)[off:]
+    y = K.gemm(x, w, bias, res, "gelu")
+    K.check_status()
+    ref = F.gelu(x.double() @ w.double().t() + bias.double(), approximate="tanh") + res.double()
+    assert ((y.double() - ref).norm() / ref.norm()).item() < TOL[dtype]
