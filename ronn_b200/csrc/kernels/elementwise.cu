@@ -520,6 +520,21 @@ __global__ void argmax_combine_kernel(const float* __restrict__ vals, const int*
   out[r] = mi;
 }
 
+// out[b] = max(1, number of j with mask[b, j] > -1e4): key lengths of an additive key-padding mask.  One launch instead of
+// compare, sum, clamp and cast (four launches of 2 to 3 us per attention node, each behind its own host call).
+template <class T>
+__global__ void key_lengths_kernel(const T* __restrict__ mask, int* __restrict__ out, int S, long ld) {
+  __shared__ float scratch[32];
+  pdl_wait();
+  pdl_trigger();
+  const T* row = mask + long(blockIdx.x) * ld;
+  const float limit = Cvt<T>::to_f(Cvt<T>::from_f(-1e4f));      // the fill value as the mask's type holds it
+  float n = 0.f;
+  for (int j = threadIdx.x; j < S; j += blockDim.x) n += Cvt<T>::to_f(row[j]) > limit ? 1.f : 0.f;
+  n = block_sum(n, scratch);                                      // exact: S < 2^24
+  if (threadIdx.x == 0) out[blockIdx.x] = n < 1.f ? 1 : int(n);
+}
+
 template <class TI, class TO>
 __global__ void cast_kernel(const TI* __restrict__ x, TO* __restrict__ y, long n) {
   const long stride = long(gridDim.x) * blockDim.x;
@@ -716,6 +731,15 @@ extern "C" int ronn_argmax(const void* x, int* idx_out, float* max_out, long row
   const int threads = cols >= 8192 ? 1024 : 256;
   if (dtype == 2) launch(argmax_kernel<float>, dim3(unsigned(rows)), dim3(threads), 0, stream, (const float*)x, idx_out, max_out, cols, ld, col_offset);
   else RONN_BY_DTYPE(dtype, launch(argmax_kernel<T>, dim3(unsigned(rows)), dim3(threads), 0, stream, (const T*)x, idx_out, max_out, cols, ld, col_offset));
+  return check_launch();
+}
+
+// mask: [rows, S] additive mask (row stride ld, unit column stride); out: int32 [rows].  dtype 0 bf16, 1 fp16.
+extern "C" int ronn_key_lengths(const void* mask, int* out, long rows, int S, long ld, int dtype, cudaStream_t stream) {
+  if (rows <= 0) return 0;
+  if (S <= 0 || S >= (1 << 24)) return -2;
+  const int threads = S >= 256 ? 256 : (S + 31) / 32 * 32;
+  RONN_BY_DTYPE(dtype, launch(key_lengths_kernel<T>, dim3(unsigned(rows)), dim3(threads), 0, stream, (const T*)mask, out, S, ld));
   return check_launch();
 }
 

@@ -36,6 +36,7 @@ def declare(lib):
     sig("ronn_swiglu_fused", [V, V, L, I, I, V])
     sig("ronn_fused_elementwise", [V, V, L, I, V, V, V, L, I, V], optional=True)
     sig("ronn_embedding", [V, V, V, V, V, L, I, I, I, L, I, V])
+    sig("ronn_key_lengths", [V, V, L, I, L, I, V])
     sig("ronn_argmax", [V, V, V, L, I, L, I, I, V])
     sig("ronn_argmax_combine", [V, V, V, I, I, V])
     sig("ronn_sample", [V, L, I, L, V, V, I, V, V, V], optional=True)

@@ -279,6 +279,18 @@ def embedding(ids: torch.Tensor, table: torch.Tensor, positions: Optional[torch.
     return out
 
 
+def key_lengths(mask: torch.Tensor) -> torch.Tensor:
+    """Visible keys per row (at least 1) of an additive key-padding mask [rows, S] in bf16 / fp16, as int32 [rows]."""
+    if mask.dim() != 2 or mask.dtype not in (torch.bfloat16, torch.float16):
+        raise KernelError("key_lengths needs a 16-bit mask [rows, S]")
+    if mask.stride(1) != 1:
+        mask = mask.contiguous()
+    out = torch.empty(mask.shape[0], dtype=torch.int32, device=mask.device)
+    _check(_native.cuda().ronn_key_lengths(mask.data_ptr(), out.data_ptr(), mask.shape[0], mask.shape[1], mask.stride(0),
+                                           _DT[mask.dtype], _stream()), "key_lengths")
+    return out
+
+
 def argmax(x: torch.Tensor, col_offset: int = 0, return_max: bool = False, out: Optional[torch.Tensor] = None):
     """Row argmax of a 2-D tensor (lowest index wins ties) as int32."""
     rows, cols = x.shape

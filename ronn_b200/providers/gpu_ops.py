@@ -160,6 +160,12 @@ class GpuOpTable:
 
         def run(i, a, c):
             x, skip = i[0], i[1]
+            if (x.dtype in _HALF and skip.dtype == x.dtype and x.shape != skip.shape and x.shape[-1] % 8 == 0
+                    and x.shape[-1] <= 32768 and not (len(i) > 4 and i[4] is not None)):
+                s = x + skip                         # a broadcast operand (position embeddings): one add, one norm launch
+                if s.shape[-1] == x.shape[-1]:
+                    return [K.layernorm(s, i[2], i[3] if len(i) > 3 else None, float(a.get("epsilon", 1e-5))), s]
+                return fallback(i, a, c)
             if (x.dtype not in _HALF or skip.dtype != x.dtype or x.shape != skip.shape or x.shape[-1] % 8
                     or x.shape[-1] > 32768 or (len(i) > 4 and i[4] is not None)):
                 return fallback(i, a, c)
@@ -285,7 +291,10 @@ class GpuOpTable:
                 q_off, k_off, v_off = 0, H, 2 * H
             if mask is not None:
                 m = mask.reshape(B, -1, mask.shape[-1])[:, 0, :] if mask.dim() > 2 else mask.reshape(B, -1)
-                kv_len = (m > -1e4).sum(dim=-1).clamp_(min=1).to(torch.int32)
+                if m.dtype in _HALF and m.device.type == "cuda" and 0 < m.shape[1] < 1 << 24:
+                    kv_len = K.key_lengths(m)
+                else:
+                    kv_len = (m > -1e4).sum(dim=-1).clamp_(min=1).to(torch.int32)
                 plan = dict(plan, kv_len=kv_len)
             out = K.dense_attention(buf, q_off, k_off, v_off, plan, heads, heads, d, causal, plan["q_len"], S)
             return [out.view(B, S, H)]
