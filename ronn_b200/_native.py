@@ -95,6 +95,7 @@ def host():
         for name in ("state", "num_tokens", "prompt_len", "preemptions", "num_computed"):
             _sig(lib, f"ronn_sched_{name}", I32, [V, I64])
         _sig(lib, "ronn_sched_get_tokens", I32, [V, I64, c_i32p, I32])
+        _sig(lib, "ronn_sched_stage_sampling", I32, [V, V, I32, V, V, I32])
         _sig(lib, "ronn_sched_get_blocks", I32, [V, I64, c_i32p, I32])
         _sig(lib, "ronn_sched_get_cpu_blocks", I32, [V, I64, c_i32p, I32])
         _sig(lib, "ronn_sched_forget", None, [V, I64])

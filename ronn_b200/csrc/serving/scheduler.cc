@@ -583,6 +583,39 @@ int32_t ronn_sched_get_tokens(void* h, int64_t id, int32_t* out, int32_t cap) {
   memcpy(out, it->second.tokens.data(), size_t(n) * 4);
   return n;
 }
+// Sampling record of a row, as the device sampler reads it.
+struct SampleRecord {
+  float temperature, top_p, repeat_penalty;
+  int32_t top_k;
+  uint64_t seed;
+  int32_t n_recent, use_counter;
+};
+static_assert(sizeof(SampleRecord) == 32, "layout shared with the device sampler");
+
+// Completes the sampling records of a step.  On entry records[i] holds request ids[i]'s parameters with its base seed; the
+// draw's seed becomes base * 0x100000001B3 + (tokens generated so far), and rows with a repeat penalty get their window:
+// the last 64 prompt tokens and what was generated after them, the newest `cap` of it, in recent[i * cap ..].
+// Returns 1 when some row has a window, 0 when none has, -1 for an unknown request.
+int32_t ronn_sched_stage_sampling(void* h, const int64_t* ids, int32_t n, SampleRecord* records, int32_t* recent, int32_t cap) {
+  Scheduler* s = static_cast<Scheduler*>(h);
+  int32_t any = 0;
+  for (int32_t i = 0; i < n; ++i) {
+    auto it = s->reqs.find(ids[i]);
+    if (it == s->reqs.end()) return -1;
+    const Request& r = it->second;
+    SampleRecord& rec = records[i];
+    const int32_t total = int32_t(r.tokens.size());
+    rec.seed = rec.seed * 0x100000001B3ull + uint64_t(int64_t(total - r.prompt_len));
+    rec.n_recent = 0;
+    if (rec.repeat_penalty != 1.0f) {
+      const int32_t from = std::max(std::max(r.prompt_len - 64, 0), total - cap);
+      rec.n_recent = total - from;
+      memcpy(recent + size_t(i) * size_t(cap), r.tokens.data() + from, size_t(rec.n_recent) * 4);
+      any = 1;
+    }
+  }
+  return any;
+}
 int32_t ronn_sched_prompt_len(void* h, int64_t id) {
   Scheduler* s = static_cast<Scheduler*>(h);
   auto it = s->reqs.find(id);

@@ -144,6 +144,9 @@ class LLMEngine:
             from ..ops import kernels as K
             n = self.cfg.max_num_seqs
             self._samp_bytes = n * K.SAMPLE_RECORD_BYTES
+            pad = bytearray(K.SAMPLE_RECORD_BYTES)
+            K.pack_sample_params(pad, 0, 0.0, 0, 1.0, 1.0, 0, 0, use_counter=False)
+            self._samp_pad = bytes(pad)
             self._samp_host = torch.zeros(self._samp_bytes + n * self._samp_recent * 4, dtype=torch.uint8).pin_memory()
             self._samp_dev = torch.zeros_like(self._samp_host, device=self.device)
             self._samp_counters = torch.zeros(n, dtype=torch.int64, device=self.device)
@@ -392,29 +395,29 @@ class LLMEngine:
         """Fills the pinned sampling records (and the recent-token windows of rows with a repeat penalty) for the rows
         of this step and copies them to the device.  The seed of a row's draw is a function of the request's seed and
         of how many tokens it has generated, so a request samples the same tokens whatever batch it shares."""
-        from ..ops import kernels as K
+        n = min(len(req_ids), rows)
+        reqs = self.requests
+        records = [self._sample_record(reqs[i]) for i in req_ids[:n].tolist()]
+        records += [self._samp_pad] * (rows - n)                                       # padded rows
         buf = self._samp_host.numpy()
-        rec = buf[self._samp_bytes:].view(np.int32).reshape(-1, self._samp_recent)
-        any_recent = False
-        for row in range(rows):
-            if row < len(req_ids):
-                r = self.requests[int(req_ids[row])]
-                p = r.params
-                n_out = self.sched.num_tokens(r.id) - len(r.prompt_tokens)
-                base = p.seed if p.seed is not None else (self._samp_seed ^ (r.id * 0x9E3779B1))
-                n_recent = 0
-                if p.repeat_penalty != 1.0:
-                    window = (r.prompt_tokens[-64:] + r.output_tokens)[-self._samp_recent:]
-                    n_recent = len(window)
-                    rec[row, :n_recent] = window
-                    any_recent = True
-                K.pack_sample_params(buf, row, p.temperature, p.top_k, p.top_p, p.repeat_penalty,
-                                     (int(base) * 0x100000001B3 + n_out) & 0xFFFFFFFFFFFFFFFF, n_recent, use_counter=False)
-            else:
-                K.pack_sample_params(buf, row, 0.0, 0, 1.0, 1.0, 0, 0, use_counter=False)     # padded row
+        buf[:rows * len(self._samp_pad)] = np.frombuffer(b"".join(records), dtype=np.uint8)
+        ptr = self._samp_host.data_ptr()
+        any_recent = n > 0 and self.sched.stage_sampling(req_ids[:n], ptr, ptr + self._samp_bytes, self._samp_recent)
         used = self._samp_bytes + (rows * self._samp_recent * 4 if any_recent else 0)
         self._samp_dev[:used].copy_(self._samp_host[:used], non_blocking=True)
         self._h2d_sampling = used
+
+    def _sample_record(self, r: Request) -> bytes:
+        """The request's sampling record with its base seed; packed again when a parameter has changed."""
+        p = r.params
+        key = (p.temperature, p.top_k, p.top_p, p.repeat_penalty, p.seed)
+        if r._sample_record is None or r._sample_record[0] != key:
+            from ..ops import kernels as K
+            base = p.seed if p.seed is not None else (self._samp_seed ^ (r.id * 0x9E3779B1))
+            rec = bytearray(K.SAMPLE_RECORD_BYTES)
+            K.pack_sample_params(rec, 0, p.temperature, p.top_k, p.top_p, p.repeat_penalty, int(base), 0, use_counter=False)
+            r._sample_record = (key, bytes(rec))
+        return r._sample_record[1]
 
     def _sample_on_device(self, logits: torch.Tensor, rows: int) -> torch.Tensor:
         from ..ops import kernels as K

@@ -55,6 +55,7 @@ class Request:
     finished_at: Optional[float] = None
     error: Optional[str] = None
     _final_tokens: Optional[List[int]] = None
+    _sample_record: Optional[tuple] = None               # (sampling parameters, their packed record): see the engine
     _token_source: Optional[object] = None       # callable returning prompt + generated tokens while the request is live
 
     @property

@@ -161,6 +161,15 @@ class Scheduler:
         self._lib.ronn_sched_get_tokens(self._h, req_id, out.ctypes.data_as(_native.c_i32p), n)
         return out[:n].tolist()
 
+    def stage_sampling(self, req_ids: np.ndarray, records_ptr: int, recent_ptr: int, recent_cap: int) -> bool:
+        """Completes a step's sampling records (seed of the draw, window of the repeat penalty) in place; whether any row
+        has a window."""
+        ids = np.ascontiguousarray(req_ids, dtype=np.int64)
+        rc = self._lib.ronn_sched_stage_sampling(self._h, ids.ctypes.data, len(ids), records_ptr, recent_ptr, recent_cap)
+        if rc < 0:
+            raise SessionError("a request of this step is unknown to the scheduler")
+        return rc > 0
+
     def prompt_len(self, req_id: int) -> int:
         return self._lib.ronn_sched_prompt_len(self._h, req_id)
 
