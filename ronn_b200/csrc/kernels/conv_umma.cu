@@ -40,6 +40,7 @@ struct ConvShape {
   int chunks;              // R * S * C / 8   (16-byte K chunks)
   int splitk;              // K slices per output tile (> 1: fp32 partial panels, reduced by the finalize kernel)
   int kb_per;              // K blocks per slice
+  int pad_w;               // left padding (im2col form; the gather pads both sides alike)
 };
 
 // tile index -> (row tile, column tile, first K block, K blocks); K slices of one output tile are adjacent indices
@@ -359,7 +360,7 @@ struct ConvProblem {
     const int rem = m0 - img * cs.Ho * cs.Wo;
     const int oh = rem / cs.Wo;
     h0 = oh * cs.stride - cs.pad;
-    w0 = (rem - oh * cs.Wo) * cs.stride - cs.pad;
+    w0 = (rem - oh * cs.Wo) * cs.stride - cs.pad_w;
     const int tap = k / cs.C;
     c = k - tap * cs.C;
     r = tap / cs.S;
@@ -535,6 +536,35 @@ __global__ void nchw_to_s2d16_kernel(const T* __restrict__ x, T* __restrict__ y,
   }
 }
 
+// The same with two zero columns before and one after every row ([N, H/2, W/2 + 3, 16]): the four horizontal taps of an
+// output position are then 64 neighbouring values wherever it lies, and the stem's K block is one 128-byte run per position.
+template <class T>
+__global__ void nchw_to_s2d16_padded_kernel(const T* __restrict__ x, T* __restrict__ y, int C, int H, int W, long total) {
+  pdl_wait();
+  pdl_trigger();
+  const int H2 = H >> 1, WP = (W >> 1) + 3;
+  for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
+    const int xo = int(i % WP) - 2;
+    const long t = i / WP;
+    const int yo = int(t % H2);
+    const long n = t / H2;
+    alignas(16) T v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = Cvt<T>::from_f(0.f);
+    if (xo >= 0 && xo < (W >> 1)) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int dy = q >> 1, dx = q & 1;
+        for (int c = 0; c < C; ++c)
+          v[q * C + c] = x[((n * C + c) * H + (2 * yo + dy)) * long(W) + 2 * xo + dx];
+      }
+    }
+    Vec8* dst = reinterpret_cast<Vec8*>(y + i * 16);
+    dst[0] = *reinterpret_cast<const Vec8*>(v);
+    dst[1] = *reinterpret_cast<const Vec8*>(v + 8);
+  }
+}
+
 // y[n, c] = mean over HW of x[n, :, :, c]; one CTA per (n, 64-channel slab), threads split HW.
 template <class T>
 __global__ void global_avgpool_nhwc_kernel(const T* __restrict__ x, T* __restrict__ y, int HW, int C) {
@@ -631,7 +661,7 @@ extern "C" int ronn_conv2d(const void* x, const void* w, const void* bias, const
                            int dtype, float* workspace, long workspace_floats, uint32_t* status, cudaStream_t stream) {
   if (N <= 0 || (C & 7) || (Cout & 7) || R <= 0 || S <= 0 || stride <= 0) return -2;
   if (long(H) * W * C * N >= (1l << 31) || long(N) * Ho * Wo * Cout >= (1l << 31)) return -4;   // 32-bit offsets inside
-  ConvShape cs{N, H, W, C, Ho, Wo, Cout, R, S, stride, pad, dil, N * Ho * Wo, R * S * C / 8, 1, 0};
+  ConvShape cs{N, H, W, C, Ho, Wo, Cout, R, S, stride, pad, dil, N * Ho * Wo, R * S * C / 8, 1, 0, pad};
   const int Kg = R * S * C;
   const int num_kb = (cs.chunks + 7) / 8;
   const int m_tiles = (cs.M + 127) / 128;
@@ -640,7 +670,8 @@ extern "C" int ronn_conv2d(const void* x, const void* w, const void* bias, const
   CUtensorMap ma;
   const bool tap16 = C == 16 && (R * S) % 4 == 0;
   bool tma = (tap16 || (C & 63) == 0) && pad >= 0 && dil * (R - 1) < 256 && dil * (S - 1) < 256;
-  if (tma) tma = make_tmap_im2col(&ma, x, N, H, W, C, Ho, Wo, stride, pad, tap16 ? 16 : 64, PG_BM) == 0;
+  if (tma) tma = make_tmap_im2col(&ma, x, N, H, W, C, C, uint64_t(W) * C, uint64_t(H) * W * C, Ho, Wo, stride, pad, pad,
+                                  tap16 ? 16 : 64, PG_BM) == 0;
   // Tile width: as wide as the layer allows (a 32-wide MMA costs as much issue time as a 128-wide one), 256 once that still
   // gives every SM a tile.  Parallelism for layers with few output tiles comes from K slices, chosen by a small cost
   // model in units of one K block: waves x (K blocks per slice + fixed cost per tile) + the reduction pass.
@@ -697,6 +728,35 @@ extern "C" int ronn_conv2d(const void* x, const void* w, const void* bias, const
   // act 3: ReLU after the residual has been added (act 1 would apply it before)
   return ronn_splitk_finalize(workspace, cs.splitk, bias, residual, out, nullptr, nullptr, nullptr, long(cs.M), Cout, 0.f,
                               act ? 3 : 0, 0, dtype, stream);
+}
+
+// First convolution of an image network, 7x7 / stride 2 / pad 3 over NCHW x [N, C <= 4, H, W] (H and W even), as a 4x4
+// convolution over its padded space-to-depth form: w [Cout, 4, 4, 16], out NHWC [N, H/2, W/2, Cout], Cout a multiple of 8
+// from 64 on, scratch: 16-byte aligned, N * (H/2) * (W/2 + 3) * 16 values.  act 0 none, 1 ReLU.  Returns -2, with nothing
+// launched, for sizes it does not take.
+extern "C" int ronn_stem_conv(const void* x, const void* w, const void* bias, void* out, void* scratch, int N, int C, int H, int W,
+                              int Cout, int act, int dtype, uint32_t* status, cudaStream_t stream) {
+  if (N <= 0 || C < 1 || C > 4 || H <= 0 || W <= 0 || (H & 1) || (W & 1) || Cout < 64 || (Cout & 7)) return -2;
+  const int Ho = H / 2, Wo = W / 2, WP = Wo + 3;
+  const long total = long(N) * Ho * WP;
+  if (total * 16 >= (1l << 31) || long(N) * Ho * Wo * Cout >= (1l << 31)) return -2;
+  CUtensorMap ma, mw;
+  if (make_tmap_im2col(&ma, scratch, N, Ho, Wo, 64, 16, uint64_t(WP) * 16, uint64_t(Ho) * WP * 16, Ho, Wo, 1, 2, 0, 64, PG_BM) != 0)
+    return -2;
+  const int bn = Cout >= 128 ? 128 : 64;
+  if (make_tmap_2d(&mw, w, uint64_t(Cout), 256, 256, uint32_t(bn), 64, 2) != 0) return -2;
+  const int grid = int((total + 255) / 256 > 148 * 64 ? 148 * 64 : (total + 255) / 256);
+  cudaError_t err;
+  if (dtype == 0) err = launch(nchw_to_s2d16_padded_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)scratch, C, H, W, total);
+  else err = launch(nchw_to_s2d16_padded_kernel<__half>, dim3(grid), dim3(256), 0, stream, (const __half*)x, (__half*)scratch, C, H, W, total);
+  if (err != cudaSuccess) return -100;
+  const ConvShape cs{N, Ho, Wo, 64, Ho, Wo, Cout, 4, 1, 1, 2, 1, N * Ho * Wo, 32, 1, 4, 0};
+  const DenseEpilogue e{out, bias, nullptr, cs.M, Cout, Cout, 0, 0, act, 0, 1};
+  if (dtype == 0)
+    return bn == 64 ? launch_im2col<64, 4, 1, __nv_bfloat16, false>(ma, mw, cs, e, 1, status, stream)
+                    : launch_im2col<128, 3, 1, __nv_bfloat16, false>(ma, mw, cs, e, 1, status, stream);
+  return bn == 64 ? launch_im2col<64, 4, 1, __half, false>(ma, mw, cs, e, 0, status, stream)
+                  : launch_im2col<128, 3, 1, __half, false>(ma, mw, cs, e, 0, status, stream);
 }
 
 extern "C" int ronn_maxpool_nhwc(const void* x, void* y, int N, int H, int W, int C, int Ho, int Wo, int k, int stride,

@@ -70,6 +70,16 @@ def stem_conv_s2d(x_nchw, w2, bias, relu):
     """7x7 / stride 2 / pad 3 first convolution of an image network from the NCHW input: one kernel rearranges the input
     into its 2x2 space-to-depth NHWC form, the implicit-GEMM kernel then runs a 4x4 stride-1 convolution with K = 256."""
     N, C, H, W = x_nchw.shape
+    Cout, dt = w2.shape[0], 0 if x_nchw.dtype == torch.bfloat16 else 1
+    out = torch.empty((N, H // 2, W // 2, Cout), dtype=x_nchw.dtype, device=x_nchw.device)
+    scratch = torch.empty(N * (H // 2) * (W // 2 + 3) * 16, dtype=x_nchw.dtype, device=x_nchw.device)
+    rc = _native.cuda().ronn_stem_conv(x_nchw.data_ptr(), w2.data_ptr(), None if bias is None else bias.data_ptr(), out.data_ptr(),
+                                       scratch.data_ptr(), N, C, H, W, Cout, 1 if relu else 0, dt,
+                                       K.status_word(x_nchw.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+    if rc == 0:
+        return out
+    if rc != -2:                                    # -2: a size the one-call form does not take, nothing was launched
+        raise K.KernelError(f"stem_conv failed with code {rc}")
     x2 = torch.empty((N, H // 2, W // 2, 16), dtype=x_nchw.dtype, device=x_nchw.device)
     rc = _native.cuda().ronn_nchw_to_s2d16(x_nchw.data_ptr(), x2.data_ptr(), N, C, H, W,
                                            0 if x_nchw.dtype == torch.bfloat16 else 1,

@@ -45,3 +45,21 @@ def test_conv_against_64_bits(shape, dtype):
     y = conv2d_nhwc(x, w, b, res, stride, pad, dil, True, out_hw=hw)
     K.check_status()
     assert ((y.double() - ref).norm() / ref.norm()).item() < tol
+
+
+# 7x7 / stride 2 / pad 3 from NCHW: narrow and wide images, every channel count the rearranged form holds, one and two column
+# tiles, and (40 channels out) the two-call form
+@pytest.mark.parametrize("shape", [(1, 3, 224, 224, 64), (2, 4, 18, 30, 64), (3, 1, 2, 2, 72), (5, 3, 160, 256, 136), (2, 3, 20, 22, 40)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_stem_against_64_bits(shape, dtype):
+    from ronn_b200.ops import kernels as K
+    from ronn_b200.providers.gpu_conv import stem_conv_s2d, stem_weights_s2d
+    N, C, H, W, Cout = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    x = torch.randn(N, C, H, W, generator=g, device="cuda").to(dtype)
+    w = (torch.randn(Cout, C, 7, 7, generator=g, device="cuda") / (49 * C) ** 0.5).to(dtype)
+    b = torch.randn(Cout, generator=g, device="cuda").to(dtype)
+    y = stem_conv_s2d(x, stem_weights_s2d(w.permute(0, 2, 3, 1).contiguous()), b, True)
+    K.check_status()
+    ref = F.relu(F.conv2d(x.double(), w.double(), b.double(), 2, 3)).permute(0, 2, 3, 1)
+    assert y.shape == ref.shape and ((y.double() - ref).norm() / ref.norm()).item() < (2 ** -8 if dtype == torch.bfloat16 else 2 ** -11)
