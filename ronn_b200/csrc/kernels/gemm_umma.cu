@@ -13,6 +13,7 @@
 #include "common.cuh"
 #include "gemm_epilogue.cuh"
 #include "tma_desc.cuh"
+#include "umma_pair.cuh"
 #include "umma_persistent.cuh"
 
 namespace ronn {
@@ -71,6 +72,68 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
 static int sm_count() { return device_sm_count(); }
 
+// The same problem on CTA pairs: tiles of 256 x BN, M index fastest.
+template <int BN, class T>
+struct DensePairProblem {
+  static constexpr bool kConstB = true;
+  const CUtensorMap* map_a;
+  const CUtensorMap* map_b;
+  PairOut out;
+  int m_tiles, n_tiles, num_kb;
+
+  __device__ __forceinline__ float row_scale(int) const { return 1.f; }
+  __device__ __forceinline__ int num_tiles() const { return m_tiles * n_tiles; }
+  __device__ __forceinline__ void tile(int t, int& m0, int& n0) const {
+    const int n = t / m_tiles;
+    m0 = (t - n * m_tiles) * 256;
+    n0 = n * BN;
+  }
+  __device__ __forceinline__ void load_a(uint8_t* smem, uint32_t bar, int k, int m) const { tma_load_2d_pair(smem, map_a, bar, k, m); }
+  __device__ __forceinline__ void load_b(uint8_t* smem, uint32_t bar, int k, int n) const { tma_load_2d_pair(smem, map_b, bar, k, n); }
+};
+
+template <int BN, int STAGES, class T>
+__global__ void __launch_bounds__(PP_THREADS)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                 const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_r, DenseEpilogue epi,
+                 int by_tma, int K, uint32_t idesc, uint32_t* status) {
+  extern __shared__ uint8_t dyn_smem[];
+  DensePairProblem<BN, T> prob{&map_a, &map_b, {&map_c, &map_r, epi, by_tma}, (epi.M + 255) / 256, (epi.N + BN - 1) / BN, (K + 63) / 64};
+  gemm_pair<BN, STAGES, 0, T>(dyn_smem, prob, idesc, status);
+}
+
+template <int BN, int STAGES, class T>
+static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, DenseEpilogue epi, int M, int N, int K, int is_bf16,
+                       uint32_t* status, cudaStream_t stream) {
+  using L = PairSmem<BN, STAGES>;
+  auto kern = gemm_pair_kernel<BN, STAGES, T>;
+  static bool configured[MAX_DEVICES] = {false};
+  if (first_use_on_device(configured)) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN_SMEM) != cudaSuccess) return -10;
+  }
+  CUtensorMap mc = ma, mr = ma;
+  const int by_tma = pair_out_maps(epi, 2, &mc, &mr);
+  const int tiles = ((N + BN - 1) / BN) * ((M + 255) / 256), pairs = sm_count() / 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * unsigned(tiles < pairs ? tiles : pairs));
+  cfg.blockDim = dim3(PP_THREADS);
+  cfg.dynamicSmemBytes = size_t(L::DYN_SMEM);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  prefer_max_shared(reinterpret_cast<const void*>(kern));
+  const uint32_t idesc = umma_idesc(256, BN, is_bf16 ? 1u : 0u, 1u);
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kern, ma, mb, mc, mr, epi, by_tma, K, idesc, status);
+  return (err == cudaSuccess && cudaGetLastError() == cudaSuccess) ? 0 : -11;
+}
+
 template <int BN, int STAGES, class T, int KA = 1>
 static int launch_dense(const CUtensorMap& ma, const CUtensorMap& mb, DenseEpilogue epi, int M, int N, int K,
                         int is_bf16, uint32_t* status, cudaStream_t stream, int splitk = 1) {
@@ -103,6 +166,39 @@ int pick_bn(int M, int N) {
   return 32;
 }
 
+// Tile form of a call with many rows (M >= 1024): the cheapest of four by a model in microseconds, fitted to chains inside
+// a CUDA graph (bf16, M 1024 to 8192, N 768 to 4096, K 768 to 4096; it names the fastest form or one within 6 % of it).
+// Every form pays a fixed part (dependency, set-up, first loads, last epilogue) and per wave of tiles the longer of its
+// main loop and its epilogue:
+//   one-CTA 128 x 256   9.0 + waves x max(0.40 per K block, 5.5; 7.0 with residual, 8.0 with GELU)
+//   pair 256 x 256      7.5 + waves x (0.6 + 0.40 per K block + 0.5 with GELU)
+//   one-CTA 128 x 128   5.5 + waves x (0.2 + 0.30 per K block + 0.5 with residual or GELU), one CTA per SM
+//   one-CTA 128 x 64    5.2 + 0.245 per K block while every SM has at most one tile, else 5 + waves x 0.42 per K block, two per SM
+// Measured, pair / 128 x 256 / 128 x 128 (us): 8192 x 3072 x 768 GELU 43.4 / 55.0 / 52.7; 8192 x 768 x 768 residual 18.7 /
+// 22.1 / 18.5; 8192 x 4096 x 1024 GELU 60.1 / 67.9 / 78.6; 4662 x 1024 x 1024 residual 20.8 / 16.5 / 17.0; 4662 x 50257 x
+// 768 (rows off the 16-byte grid) 412 / 627.
+enum TileForm { FORM_64, FORM_128, FORM_256, FORM_PAIR };
+static TileForm pick_form(int M, int N, int K, int act, bool residual, bool out_fp32) {
+  const int sms = sm_count();
+  const long mt = (M + 127) / 128, mt2 = (M + 255) / 256;
+  const float kb = float((K + 63) / 64);
+  auto waves = [](long tiles, int slots) { return float((tiles + slots - 1) / slots); };
+  const bool gelu = act == 2;
+  const long t64 = mt * ((N + 63) / 64);
+  TileForm best = FORM_64;
+  float cost = t64 <= sms ? 5.2f + 0.245f * kb : 5.f + waves(t64, 2 * sms) * 0.42f * kb;
+  auto offer = [&](TileForm f, float c) {
+    if (c < cost) { cost = c; best = f; }
+  };
+  offer(FORM_128, 5.5f + waves(mt * ((N + 127) / 128), sms) * (0.2f + 0.30f * kb + (gelu || residual ? 0.5f : 0.f)));
+  if (N > 128) {
+    const float epi = gelu ? 8.f : (residual || out_fp32 ? 7.f : 5.5f);
+    offer(FORM_256, 9.f + waves(mt * ((N + 255) / 256), sms) * (0.40f * kb > epi ? 0.40f * kb : epi));
+    if (!out_fp32) offer(FORM_PAIR, 7.5f + waves(mt2 * ((N + 255) / 256), sms / 2) * (0.6f + 0.40f * kb + (gelu ? 0.5f : 0.f)));
+  }
+  return best;
+}
+
 // Pipeline depth.  A CTA that is alone on its SM is fed by the bytes it keeps in flight, so when the whole problem
 // is at most one CTA per SM the ring is twice as deep (6 / 8 / 10 stages for BN 128 / 64 / 32, one CTA per SM)
 // instead of two co-resident CTAs with half the ring each.  bn | 0x1000 forces the deep ring, bn | 0x2000 the shallow.
@@ -127,7 +223,7 @@ extern "C" int ronn_gemm_skinny(const void* A, const void* W, void* C, const voi
                                 const void* gamma, const void* beta, float eps, int norm, int M, int N, int K, long lda,
                                 long ldw, long ldc, int dtype, int act, int out_fp32, cudaStream_t stream);
 
-// dtype: 0 = bf16, 1 = fp16.  act: 0 none, 1 relu, 2 gelu.  bn: 0 = auto, else 32|64|128|256 (| 0x1000 deep ring,
+// dtype: 0 = bf16, 1 = fp16.  act: 0 none, 1 relu, 2 gelu.  bn: 0 = auto, else 32|64|128|256, or 256 | 0x4000 for CTA pairs (| 0x1000 deep ring,
 // | 0x2000 shallow ring; default picks by tile count).
 // lda/ldw/ldc in elements; K and the leading dimensions must be multiples of 8.
 // Returns 0 on success, negative on configuration errors.
@@ -139,7 +235,15 @@ extern "C" int ronn_gemm(const void* A, const void* W, void* C, const void* bias
   if (bn == 0 && skinny_rule(M, N, K))
     return ronn_gemm_skinny(A, W, C, bias, residual, nullptr, nullptr, 0.f, 0, M, N, K, lda, ldw, ldc, dtype, act, out_fp32, stream);
   int deep = deep_mode(bn);
+  bool pair = (bn & 0x4000) != 0;
   bn &= 0xfff;
+  if (bn == 0 && M >= 1024) {
+    const TileForm f = pick_form(M, N, K, act, residual != nullptr, out_fp32 != 0);
+    pair = f == FORM_PAIR;
+    bn = f == FORM_64 ? 64 : (f == FORM_128 ? 128 : 256);
+    if (f == FORM_128) deep = 1;
+    if (f == FORM_64) deep = 0;
+  }
   if (bn == 0) bn = pick_bn(M, N);
   if (deep < 0) deep = wants_deep(M, N, bn, 1);
   // rows off the 16-byte grid leave through the store-staging area, which only the deep rings carry
@@ -147,10 +251,18 @@ extern "C" int ronn_gemm(const void* A, const void* W, void* C, const void* bias
   CUtensorMap ma, mb;
   int rc = make_tmap_2d(&ma, A, uint64_t(M), uint64_t(K), uint64_t(lda), PG_BM, 64, 2);
   if (rc) return rc - 20;
-  rc = make_tmap_2d(&mb, W, uint64_t(N), uint64_t(K), uint64_t(ldw), uint32_t(bn), 64, 2);
+  rc = make_tmap_2d(&mb, W, uint64_t(N), uint64_t(K), uint64_t(ldw), uint32_t(pair ? bn / 2 : bn), 64, 2);
   if (rc) return rc - 30;
   DenseEpilogue e{C, bias, residual, M, N, ldc, 0, 0, act, out_fp32};
   const int bf = dtype == 0;
+#define RONN_PAIR(BN_, ST_)                                                                           \
+  return bf ? launch_pair<BN_, ST_, __nv_bfloat16>(ma, mb, e, M, N, K, 1, status, stream)             \
+            : launch_pair<BN_, ST_, __half>(ma, mb, e, M, N, K, 0, status, stream)
+  if (pair) {
+    if (bn == 256) RONN_PAIR(256, 5);
+    return -3;
+  }
+#undef RONN_PAIR
 #define RONN_DISPATCH(BN_, ST_, KA_)                                                                  \
   return bf ? launch_dense<BN_, ST_, __nv_bfloat16, KA_>(ma, mb, e, M, N, K, 1, status, stream)       \
             : launch_dense<BN_, ST_, __half, KA_>(ma, mb, e, M, N, K, 0, status, stream)

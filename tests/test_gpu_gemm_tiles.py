@@ -41,3 +41,34 @@ def test_bias_and_residual_alignment(M, N, Kd, off, dtype):
     K.check_status()
     ref = F.gelu(x.double() @ w.double().t() + bias.double(), approximate="tanh") + res.double()
     assert ((y.double() - ref).norm() / ref.norm()).item() < TOL[dtype]
+
+
+# CTA pairs: rows past the second half of a tile, columns cut inside a box and inside a tile, one and several K blocks, results
+# on and off the 16-byte grid, more tiles than pairs
+@pytest.mark.parametrize("M,N,Kd", [(256, 256, 64), (129, 200, 72), (300, 1000, 128), (1, 264, 8), (1000, 515, 320), (5200, 2304, 64)])
+@pytest.mark.parametrize("act", ["", "relu", "gelu"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_cta_pairs(M, N, Kd, act, dtype):
+    from ronn_b200.ops import kernels as K
+    x, w, bias, res = _operands(M, N, Kd, dtype)
+    lin = x.double() @ w.double().t() + bias.double()
+    ref = {"": lin, "relu": F.relu(lin), "gelu": F.gelu(lin, approximate="tanh")}[act]
+    for r in (None, res):
+        out = torch.full((M + 1, N), 7.0, dtype=dtype, device="cuda")
+        K.gemm(x, w, bias, r, act, out=out[:M], bn=0x4000 | 256)
+        K.check_status()
+        want = ref if r is None else ref + r.double()
+        assert ((out[:M].double() - want).norm() / want.norm()).item() < TOL[dtype] and bool((out[M] == 7).all())
+    y32 = K.gemm(x, w, None, None, "", out_fp32=True, bn=0x4000 | 256)
+    assert ((y32.double() - x.double() @ w.double().t()).norm() / y32.double().norm()).item() < 1e-5
+
+
+# the automatic choice over sizes that end in each of its forms
+@pytest.mark.parametrize("M,N,Kd", [(1024, 768, 768), (2048, 768, 3072), (4662, 1024, 1024), (8192, 3072, 768), (1024, 96, 64)])
+def test_automatic_forms_agree(M, N, Kd):
+    from ronn_b200.ops import kernels as K
+    x, w, bias, res = _operands(M, N, Kd, torch.bfloat16)
+    want = F.gelu(x.double() @ w.double().t() + bias.double(), approximate="tanh") + res.double()
+    y = K.gemm(x, w, bias, res, "gelu")
+    K.check_status()
+    assert ((y.double() - want).norm() / want.norm()).item() < TOL[torch.bfloat16]
