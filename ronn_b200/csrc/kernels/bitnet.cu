@@ -16,6 +16,7 @@
 #include "ptx_sm100.cuh"
 #include "rowwise_stream.h"
 #include "tma_desc.cuh"
+#include "umma_pair.cuh"
 
 namespace ronn {
 
@@ -556,6 +557,56 @@ bitlinear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   }
 }
 
+// ---------------------------------------------------------------------------------------- many rows: expand once, dense int8
+// With thousands of rows every 128 x 128 tile of the kernel above expands its weight tile again (64 times over at 8192
+// rows) and the expander warps set the pace.  There the packed matrix is expanded once into int8 scratch, 1.25 bytes of
+// traffic per weight, and the product runs as a dense int8 GEMM on CTA pairs.  Same integers, same scaling: same results.
+// 8192 rows, us before / after: N 7680 K 2560 347 / 120, N 13824 K 2560 622 / 215, N 2560 K 6912 256 / 113; 1024 rows:
+// 54 / 29, 81 / 42, 58 / 32.
+__global__ void ternary_expand_kernel(const uint4* __restrict__ packed, int4* __restrict__ out, long n16) {
+  pdl_wait();                                    // the scratch may belong to the previous kernel of the stream until it ends
+  pdl_trigger();
+  const long stride = long(gridDim.x) * blockDim.x;
+  for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n16; i += stride) {
+    const uint4 w = packed[i];
+    out[i * 4] = expand16(w.x);
+    out[i * 4 + 1] = expand16(w.y);
+    out[i * 4 + 2] = expand16(w.z);
+    out[i * 4 + 3] = expand16(w.w);
+  }
+}
+
+template <int BN, class T>
+struct BitPairProblem {
+  static constexpr bool kConstB = false;         // written by the expansion just before
+  const CUtensorMap* map_a;
+  const CUtensorMap* map_b;
+  const float* x_scale;
+  float w_scale;
+  PairOut out;
+  int m_tiles, n_tiles, num_kb;
+
+  __device__ __forceinline__ float row_scale(int m) const { return m < out.e.M ? x_scale[m] * w_scale : 0.f; }
+  __device__ __forceinline__ int num_tiles() const { return m_tiles * n_tiles; }
+  __device__ __forceinline__ void tile(int t, int& m0, int& n0) const {
+    const int n = t / m_tiles;
+    m0 = (t - n * m_tiles) * 256;
+    n0 = n * BN;
+  }
+  __device__ __forceinline__ void load_a(uint8_t* smem, uint32_t bar, int k, int m) const { tma_load_2d_pair(smem, map_a, bar, k, m); }
+  __device__ __forceinline__ void load_b(uint8_t* smem, uint32_t bar, int k, int n) const { tma_load_2d_pair(smem, map_b, bar, k, n); }
+};
+
+template <int BN, int STAGES, class T>
+__global__ void __launch_bounds__(PP_THREADS)
+bitlinear_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                      const __grid_constant__ CUtensorMap map_c, const float* x_scale, float w_scale, DenseEpilogue epi,
+                      int by_tma, int K, uint32_t idesc, uint32_t* status) {
+  extern __shared__ uint8_t dyn_smem[];
+  BitPairProblem<BN, T> prob{&map_a, &map_b, x_scale, w_scale, {&map_c, &map_c, epi, by_tma}, (epi.M + 255) / 256, (epi.N + BN - 1) / BN, (K + 127) / 128};
+  gemm_pair<BN, STAGES, 1, T>(dyn_smem, prob, idesc, status);
+}
+
 // Offline packing on the device: int8 values in {-1,0,1} [rows, K] -> [rows, K/4] codes.
 __global__ void ternary_pack_kernel(const int8_t* __restrict__ v, uint8_t* __restrict__ packed, long rows, int K) {
   const long total = rows * (K >> 2);
@@ -569,6 +620,49 @@ __global__ void ternary_pack_kernel(const int8_t* __restrict__ v, uint8_t* __res
     }
     packed[i] = uint8_t(b);
   }
+}
+
+template <class T>
+static int launch_bitlinear_pair(const void* xq, const void* w_packed, const float* xs, float ws, const void* bias, void* out, int M,
+                                 int N, int K, int ldx, uint32_t* status, cudaStream_t stream, void* workspace) {
+  constexpr int BN = 256, STAGES = 5;
+  using L = PairSmem<BN, STAGES>;
+  auto kern = bitlinear_pair_kernel<BN, STAGES, T>;
+  static bool configured[MAX_DEVICES] = {false};
+  if (first_use_on_device(configured)) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN_SMEM) != cudaSuccess) return -10;
+  }
+  CUtensorMap ma, mb;
+  int rc = make_tmap_2d(&ma, xq, uint64_t(M), uint64_t(K), uint64_t(ldx), 128, 128, 1);
+  if (rc) return rc - 20;
+  rc = make_tmap_2d(&mb, workspace, uint64_t(N), uint64_t(K), uint64_t(K), BN / 2, 128, 1);
+  if (rc) return rc - 30;
+  const long n16 = long(N) * K / 64;
+  const long blocks = (n16 + 255) / 256, cap = long(device_sm_count()) * 16;
+  cudaError_t err = launch(ternary_expand_kernel, dim3(unsigned(blocks < cap ? blocks : cap)), dim3(256), 0, stream,
+                           static_cast<const uint4*>(w_packed), static_cast<int4*>(workspace), n16);
+  if (err != cudaSuccess) return -11;
+  const int tiles = ((N + BN - 1) / BN) * ((M + 255) / 256), pairs = device_sm_count() / 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * unsigned(tiles < pairs ? tiles : pairs));
+  cfg.blockDim = dim3(PP_THREADS);
+  cfg.dynamicSmemBytes = size_t(L::DYN_SMEM);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  prefer_max_shared(reinterpret_cast<const void*>(kern));
+  const DenseEpilogue e{out, bias, nullptr, M, N, N, 0, 0, 0, 0, 0};
+  CUtensorMap mc = ma, mr = ma;
+  const int by_tma = pair_out_maps(e, 2, &mc, &mr);
+  err = cudaLaunchKernelEx(&cfg, kern, ma, mb, mc, xs, ws, e, by_tma, K, umma_idesc(256, BN, 1u, 2u), status);
+  return (err == cudaSuccess && cudaGetLastError() == cudaSuccess) ? 0 : -11;
 }
 
 template <int BN, class T, bool WTMA>
@@ -678,10 +772,17 @@ static void bitlinear_plan(int M, int N, int K, bool may_slice, int& bn, int& S)
   }
 }
 
-// Bytes of scratch memory a call of this shape wants for its K slices (0: the shape is not sliced).  At most one CTA
-// per SM is sliced, so the answer never exceeds 148 x 64 KB.
+// Whether the weights are worth expanding once for the whole call: from BL_EXPAND_ROWS rows on (about twice as fast there;
+// at 512 rows the tiles of the other kernel still fit two waves), when the packed rows are whole 16-byte pieces (K a
+// multiple of 64).
+constexpr int BL_EXPAND_ROWS = 1024;
+static bool bitlinear_expands(int M, int K) { return M >= BL_EXPAND_ROWS && (K & 63) == 0; }
+
+// Bytes of scratch memory a call of this shape wants: for the expanded weights of a call with many rows (one byte per
+// weight), or for its K slices (at most one CTA per SM is sliced, so never above 148 x 64 KB); 0: none.
 extern "C" long ronn_bitlinear_workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (bitlinear_expands(M, K)) return long(N) * K;
   int bn, S;
   bitlinear_plan(M, N, K, true, bn, S);
   if (S == 1) return 0;
@@ -710,8 +811,12 @@ static int bitlinear_impl(const void* xq, const void* w_packed, const float* x_s
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   if ((K & 15) || (ldx & 15)) return -2;
   if (reinterpret_cast<uintptr_t>(workspace) & 15) return -2;
+  if (workspace != nullptr && slot_state == nullptr && bitlinear_expands(M, K) && (reinterpret_cast<uintptr_t>(w_packed) & 15) == 0)
+    return dtype == 0 ? launch_bitlinear_pair<__nv_bfloat16>(xq, w_packed, x_scale, w_scale, bias, out, M, N, K, ldx, status, stream, workspace)
+                      : launch_bitlinear_pair<__half>(xq, w_packed, x_scale, w_scale, bias, out, M, N, K, ldx, status, stream, workspace);
   int bn, S;
-  bitlinear_plan(M, N, K, workspace != nullptr, bn, S);
+  // scratch that was sized for expanded weights is not used for K slices
+  bitlinear_plan(M, N, K, workspace != nullptr && !bitlinear_expands(M, K), bn, S);
   CUtensorMap mx;
   int rc = make_tmap_2d(&mx, xq, uint64_t(M), uint64_t(K), uint64_t(ldx), 128, 128, 1);
   if (rc) return rc - 20;
