@@ -672,25 +672,51 @@ extern "C" int ronn_conv2d(const void* x, const void* w, const void* bias, const
   bool tma = (tap16 || (C & 63) == 0) && pad >= 0 && dil * (R - 1) < 256 && dil * (S - 1) < 256;
   if (tma) tma = make_tmap_im2col(&ma, x, N, H, W, C, C, uint64_t(W) * C, uint64_t(H) * W * C, Ho, Wo, stride, pad, pad,
                                   tap16 ? 16 : 64, PG_BM) == 0;
-  // Tile width: as wide as the layer allows (a 32-wide MMA costs as much issue time as a 128-wide one), 256 once that still
-  // gives every SM a tile.  Parallelism for layers with few output tiles comes from K slices, chosen by a small cost
-  // model in units of one K block: waves x (K blocks per slice + fixed cost per tile) + the reduction pass.
   int bn = Cout >= 128 ? 128 : (Cout >= 64 ? 64 : 32);
   if (tma && bn < 64) tma = false;
-  if (tma && !tap16 && Cout % 256 == 0 && m_tiles * (Cout / 256) >= 148) bn = 256;
-  const int tiles = m_tiles * ((Cout + bn - 1) / bn);
-  const int resident = device_sm_count() * (bn == 64 || bn == 32 || (tma && bn == 128) ? 2 : 1);
   int splitk = 1;
-  if (workspace != nullptr) {
-    int best = 1 << 30;
-    for (int sk = 1; sk <= 16; ++sk) {
-      if (sk > 1 && (num_kb / sk < 4 || long(sk) * cs.M * Cout > workspace_floats)) break;
-      const int waves = (tiles * sk + resident - 1) / resident;
-      const int cost = waves * ((num_kb + sk - 1) / sk + 6) + (sk > 1 ? 8 : 0);
-      if (cost < best) { best = cost; splitk = sk; }
+  if (tma && !tap16) {
+    // Tile width and number of K slices: the cheapest by the microsecond model of the dense GEMM's forms (one main loop):
+    // 256 and 128 wide with one CTA per SM, 64 wide with two; every wave pays its K blocks or, if longer, its epilogue.
+    // K slices add the reduction kernel (3 us) and their fp32 panels, written and read at about 3 TB/s.  A model in K blocks
+    // with a fixed price for the reduction sliced layers that one wave held anyway: 3x3 128 -> 256 / 2 at 28 x 28, batch 32:
+    // 25 us with three slices.
+    const int sms = device_sm_count();
+    float best = 1e30f;
+    const int widths[3] = {256, 128, 64};
+    for (int i = 0; i < 3; ++i) {
+      const int w = widths[i];
+      if (w > 64 && Cout < w) continue;
+      const long tiles = long(m_tiles) * ((Cout + w - 1) / w);
+      for (int sk = 1; sk <= 16; ++sk) {
+        if (sk > 1 && (workspace == nullptr || num_kb / sk < 4 || long(sk) * cs.M * Cout > workspace_floats)) break;
+        const float kb = float((num_kb + sk - 1) / sk);
+        const long n = tiles * sk;
+        float t;
+        if (w == 256) t = 9.f + float((n + sms - 1) / sms) * (0.40f * kb > 6.5f ? 0.40f * kb : 6.5f);
+        else if (w == 128) t = 5.5f + float((n + sms - 1) / sms) * (0.7f + 0.30f * kb);
+        else t = n <= sms ? 5.2f + 0.245f * kb : 5.f + float((n + 2 * sms - 1) / (2 * sms)) * (0.42f * kb > 3.f ? 0.42f * kb : 3.f);
+        if (sk > 1) t += 3.f + float(sk) * float(cs.M) * float(Cout) * 8.f / 3e6f;
+        if (t < best) { best = t; bn = w; splitk = sk; }
+      }
     }
-  } else if (!tma) {
-    while (bn > 32 && m_tiles * ((Cout + bn - 1) / bn) < 148) bn >>= 1;
+  } else {
+    // Tile width: as wide as the layer allows (a 32-wide MMA costs as much issue time as a 128-wide one).  Parallelism for
+    // layers with few output tiles comes from K slices, chosen by a small cost model in units of one K block: waves x (K
+    // blocks per slice + fixed cost per tile) + the reduction pass.
+    const int tiles = m_tiles * ((Cout + bn - 1) / bn);
+    const int resident = device_sm_count() * (bn >= 128 && !tap16 ? 1 : 2);
+    if (workspace != nullptr) {
+      int best = 1 << 30;
+      for (int sk = 1; sk <= 8; ++sk) {
+        if (sk > 1 && (num_kb / sk < 6 || long(sk) * cs.M * Cout > workspace_floats)) break;
+        const int waves = (tiles * sk + resident - 1) / resident;
+        const int cost = waves * ((num_kb + sk - 1) / sk + 6) + (sk > 1 ? 8 : 0);
+        if (cost < best) { best = cost; splitk = sk; }
+      }
+    } else if (!tma) {
+      while (bn > 32 && m_tiles * ((Cout + bn - 1) / bn) < 148) bn >>= 1;
+    }
   }
   cs.kb_per = (num_kb + splitk - 1) / splitk;
   cs.splitk = (num_kb + cs.kb_per - 1) / cs.kb_per;
@@ -704,15 +730,14 @@ extern "C" int ronn_conv2d(const void* x, const void* w, const void* bias, const
                                : launch_conv<BN_, __half>(x, mw, cs, e, 0, status, stream)
 #define RONN_IM2COL(BN_, ST_, KA_, TAP_) rc = bf ? launch_im2col<BN_, ST_, KA_, __nv_bfloat16, TAP_>(ma, mw, cs, e, 1, status, stream) \
                                                 : launch_im2col<BN_, ST_, KA_, __half, TAP_>(ma, mw, cs, e, 0, status, stream)
-  // few tiles: one CTA per SM with a deep ring of two-atom stages, as in the dense GEMM
-  const bool deep = tiles * cs.splitk <= device_sm_count();
+  // 128 wide, or few tiles: one CTA per SM with a deep ring of two-atom stages, as in the dense GEMM
+  const bool deep = bn == 128 || m_tiles * ((Cout + bn - 1) / bn) * cs.splitk <= device_sm_count();
   if (tma && tap16) {
     if (bn == 64) RONN_IM2COL(64, 4, 1, true);
     else RONN_IM2COL(128, 3, 1, true);
   } else if (tma) {
     if (bn == 256) RONN_IM2COL(256, 4, 1, false);
-    else if (bn == 128 && deep) RONN_IM2COL(128, 3, 2, false);
-    else if (bn == 128) RONN_IM2COL(128, 3, 1, false);
+    else if (bn == 128) RONN_IM2COL(128, 3, 2, false);
     else if (deep) RONN_IM2COL(64, 4, 2, false);
     else RONN_IM2COL(64, 4, 1, false);
   } else {
