@@ -334,7 +334,9 @@ static int launch_conv(const void* x, const CUtensorMap& mw, const ConvShape& cs
 // each a tile of 128 rows x 32 bytes.
 template <int BN, class T, bool TAP16>
 struct ConvProblem {
-  static constexpr bool kForceStage = false;
+  // results leave in 64-byte runs also from the 64-wide tiles, which gave a ring stage for it: the stem at batch 117 (188 MB of
+  // results) 155 -> 129 us with its operand as four taps per block, ResNet-18 at batch 117 885 -> 857 us, batch 32 366 -> 356
+  static constexpr bool kForceStage = true;
   static constexpr bool kTapA = TAP16;
   const CUtensorMap* map_a;
   const CUtensorMap* map_w;
@@ -422,7 +424,7 @@ conv_im2col_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 template <int BN, int STAGES, int KA, class T, bool TAP16>
 static int launch_im2col(const CUtensorMap& ma, const CUtensorMap& mw, const ConvShape& cs, const DenseEpilogue& e, int is_bf16,
                          uint32_t* status, cudaStream_t stream) {
-  using L = PGemmSmem<BN, STAGES, false, KA>;
+  using L = PGemmSmem<BN, STAGES, true, KA>;
   auto kern = conv_im2col_kernel<BN, STAGES, KA, T, TAP16>;
   static bool configured[MAX_DEVICES] = {false};
   if (first_use_on_device(configured)) {
@@ -733,13 +735,13 @@ extern "C" int ronn_conv2d(const void* x, const void* w, const void* bias, const
   // 128 wide, or few tiles: one CTA per SM with a deep ring of two-atom stages, as in the dense GEMM
   const bool deep = bn == 128 || m_tiles * ((Cout + bn - 1) / bn) * cs.splitk <= device_sm_count();
   if (tma && tap16) {
-    if (bn == 64) RONN_IM2COL(64, 4, 1, true);
-    else RONN_IM2COL(128, 3, 1, true);
+    if (bn == 64) RONN_IM2COL(64, 3, 1, true);
+    else RONN_IM2COL(128, 3, 2, true);
   } else if (tma) {
     if (bn == 256) RONN_IM2COL(256, 4, 1, false);
     else if (bn == 128) RONN_IM2COL(128, 3, 2, false);
     else if (deep) RONN_IM2COL(64, 4, 2, false);
-    else RONN_IM2COL(64, 4, 1, false);
+    else RONN_IM2COL(64, 3, 1, false);
   } else {
     switch (bn) {
       case 128: RONN_CONV(128); break;
@@ -778,10 +780,10 @@ extern "C" int ronn_stem_conv(const void* x, const void* w, const void* bias, vo
   const ConvShape cs{N, Ho, Wo, 64, Ho, Wo, Cout, 4, 1, 1, 2, 1, N * Ho * Wo, 32, 1, 4, 0};
   const DenseEpilogue e{out, bias, nullptr, cs.M, Cout, Cout, 0, 0, act, 0, 1};
   if (dtype == 0)
-    return bn == 64 ? launch_im2col<64, 4, 1, __nv_bfloat16, false>(ma, mw, cs, e, 1, status, stream)
-                    : launch_im2col<128, 3, 1, __nv_bfloat16, false>(ma, mw, cs, e, 1, status, stream);
-  return bn == 64 ? launch_im2col<64, 4, 1, __half, false>(ma, mw, cs, e, 0, status, stream)
-                  : launch_im2col<128, 3, 1, __half, false>(ma, mw, cs, e, 0, status, stream);
+    return bn == 64 ? launch_im2col<64, 3, 1, __nv_bfloat16, false>(ma, mw, cs, e, 1, status, stream)
+                    : launch_im2col<128, 3, 2, __nv_bfloat16, false>(ma, mw, cs, e, 1, status, stream);
+  return bn == 64 ? launch_im2col<64, 3, 1, __half, false>(ma, mw, cs, e, 0, status, stream)
+                  : launch_im2col<128, 3, 2, __half, false>(ma, mw, cs, e, 0, status, stream);
 }
 
 extern "C" int ronn_maxpool_nhwc(const void* x, void* y, int N, int H, int W, int C, int Ho, int Wo, int k, int stride,
