@@ -166,7 +166,8 @@ int pick_bn(int M, int N) {
   return 32;
 }
 
-// Tile form of a call with many rows (M >= 1024): the cheapest of four by a model in microseconds, fitted to chains inside
+// Tile form of a call with many rows (M >= 1024, or fewer with columns enough for 120 tiles of 128: 768 x 4096 x 1024 GELU
+// took 23.5 us on two 128-wide CTAs per SM, 16.0 on one): the cheapest of four by a model in microseconds, fitted to chains inside
 // a CUDA graph (bf16, M 1024 to 8192, N 768 to 4096, K 768 to 4096; it names the fastest form or one within 6 % of it).
 // Every form pays a fixed part (dependency, set-up, first loads, last epilogue) and per wave of tiles the longer of its
 // main loop and its epilogue:
@@ -237,7 +238,7 @@ extern "C" int ronn_gemm(const void* A, const void* W, void* C, const void* bias
   int deep = deep_mode(bn);
   bool pair = (bn & 0x4000) != 0;
   bn &= 0xfff;
-  if (bn == 0 && M >= 1024) {
+  if (bn == 0 && (M >= 1024 || (M > 256 && pick_bn(M, N) >= 128))) {
     const TileForm f = pick_form(M, N, K, act, residual != nullptr, out_fp32 != 0);
     pair = f == FORM_PAIR;
     bn = f == FORM_64 ? 64 : (f == FORM_128 ? 128 : 256);
