@@ -21,6 +21,10 @@ class KernelError(RonnError):
     prefix = "Kernel error: "
 
 
+class OperandError(KernelError):
+    """Operands of another type, device, length or alignment than the kernel reads; nothing was launched."""
+
+
 _DT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 _ACT = {"": 0, None: 0, "none": 0, "Relu": 1, "relu": 1, "Gelu": 2, "gelu": 2}
 _STATUS = {}
@@ -112,8 +116,9 @@ def norm_gemm(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor]
     N = w_nk.shape[0]
     if not norm_gemm_ok(M, K) or w_nk.shape[1] != K or x.stride(1) != 1 or w_nk.stride(1) != 1:
         raise KernelError(f"norm_gemm does not take x {tuple(x.shape)} w {tuple(w_nk.shape)}")
-    if x.dtype not in (torch.bfloat16, torch.float16) or any(t is not None and t.dtype != x.dtype for t in (w_nk, gamma, beta, bias)):
-        raise KernelError("norm_gemm needs bf16/fp16 operands of one dtype")
+    if w_nk.dtype != x.dtype or (bias is not None and (bias.dtype != x.dtype or bias.numel() != N)):
+        raise KernelError("norm_gemm needs bf16/fp16 operands of one dtype and a bias of one value per output")
+    _check_norm_operands(x, None, gamma, beta)
     if out is None:
         out = torch.empty((M, N), dtype=x.dtype, device=x.device)
     rc = _native.cuda().ronn_gemm_skinny(x.data_ptr(), w_nk.data_ptr(), out.data_ptr(), _ptr(bias), None, gamma.data_ptr(),
@@ -124,7 +129,24 @@ def norm_gemm(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor]
     return out
 
 
+def _check_norm_operands(x, residual, *params) -> None:
+    """The norm kernels read addresses as rows and parameters of H values of x's type: refuse what is not that."""
+    H = x.shape[-1] if x.dim() else 0
+    if x.dtype not in (torch.bfloat16, torch.float16) or x.device.type != "cuda" or H % 8 or not 0 < H <= 32768:
+        raise OperandError(f"the norm kernel needs 16-bit rows of a multiple of 8 up to 32768 values on a CUDA device, got "
+                           f"{tuple(x.shape)} {x.dtype} on {x.device}")
+    for p in params:
+        if p is not None and (p.dtype != x.dtype or p.device != x.device or p.numel() != H or not p.is_contiguous()
+                              or p.data_ptr() % 16):
+            raise OperandError(f"norm parameters must be {H} values of {x.dtype} on {x.device}, contiguous from a 16-byte "
+                               f"boundary, got {tuple(p.shape)} {p.dtype} on {p.device}")
+    if residual is not None and (residual.dtype != x.dtype or residual.device != x.device or residual.numel() != x.numel()):
+        raise OperandError(f"the norm's residual must match its input, got {tuple(residual.shape)} {residual.dtype} on "
+                           f"{residual.device}")
+
+
 def _norm(x, gamma, beta, residual, eps, rms, sum_out):
+    _check_norm_operands(x, residual, gamma, beta)
     H = x.shape[-1]
     x2 = x.reshape(-1, H)
     if x2.stride(1) != 1:

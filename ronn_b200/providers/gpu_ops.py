@@ -147,41 +147,44 @@ class GpuOpTable:
         K = self.K
 
         def run(i, a, c):
-            x = i[0]
-            if x.dtype not in _HALF or x.shape[-1] % 8 or x.shape[-1] > 32768:
+            try:
+                return [K.layernorm(i[0], i[1] if len(i) > 1 else None, i[2] if len(i) > 2 else None,
+                                    float(a.get("epsilon", 1e-5)))]
+            except K.OperandError:
                 return fallback(i, a, c)
-            return [K.layernorm(x, i[1] if len(i) > 1 else None, i[2] if len(i) > 2 else None,
-                                float(a.get("epsilon", 1e-5)))]
         return run
 
     def _skip_layernorm(self, node, fallback):
-        """LayerNorm(x + skip) and the sum in one launch of the norm kernel."""
+        """LayerNorm(x + skip) and the sum in one launch of the norm kernel; with a broadcast skip (position embeddings) one
+        add and one norm launch.  What the norm kernel refuses (parameters kept in another type, operands that shape
+        arithmetic left on the host, lengths that do not match) is the library operator's to convert or refuse."""
         K = self.K
 
         def run(i, a, c):
-            x, skip = i[0], i[1]
-            if (x.dtype in _HALF and skip.dtype == x.dtype and x.shape != skip.shape and x.shape[-1] % 8 == 0
-                    and x.shape[-1] <= 32768 and not (len(i) > 4 and i[4] is not None)):
-                s = x + skip                         # a broadcast operand (position embeddings): one add, one norm launch
+            x, skip, gamma, beta = i[0], i[1], i[2], i[3] if len(i) > 3 else None
+            if x.dtype not in _HALF or skip.dtype != x.dtype or skip.device != x.device or (len(i) > 4 and i[4] is not None):
+                return fallback(i, a, c)
+            eps = float(a.get("epsilon", 1e-5))
+            try:
+                if x.shape == skip.shape:
+                    y, s = K.layernorm(x, gamma, beta, eps, residual=skip, return_sum=True)
+                    return [y, s]
+                s = x + skip
                 if s.shape[-1] == x.shape[-1]:
-                    return [K.layernorm(s, i[2], i[3] if len(i) > 3 else None, float(a.get("epsilon", 1e-5))), s]
-                return fallback(i, a, c)
-            if (x.dtype not in _HALF or skip.dtype != x.dtype or x.shape != skip.shape or x.shape[-1] % 8
-                    or x.shape[-1] > 32768 or (len(i) > 4 and i[4] is not None)):
-                return fallback(i, a, c)
-            y, s = K.layernorm(x, i[2], i[3] if len(i) > 3 else None, float(a.get("epsilon", 1e-5)), residual=skip,
-                               return_sum=True)
-            return [y, s]
+                    return [K.layernorm(s, gamma, beta, eps), s]
+            except K.OperandError:
+                pass
+            return fallback(i, a, c)
         return run
 
     def _rmsnorm(self, node, fallback):
         K = self.K
 
         def run(i, a, c):
-            x = i[0]
-            if x.dtype not in _HALF or x.shape[-1] % 8:
+            try:
+                return [K.rmsnorm(i[0], i[1], float(a.get("epsilon", 1e-5)))]
+            except K.OperandError:
                 return fallback(i, a, c)
-            return [K.rmsnorm(x, i[1], float(a.get("epsilon", 1e-5)))]
         return run
 
     def _softmax(self, node, fallback):
