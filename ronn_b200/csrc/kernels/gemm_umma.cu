@@ -202,18 +202,44 @@ static TileForm pick_form(int M, int N, int K, int act, bool residual, bool out_
 
 // Pipeline depth.  A CTA that is alone on its SM is fed by the bytes it keeps in flight, so when the whole problem
 // is at most one CTA per SM the ring is twice as deep (6 / 8 / 10 stages for BN 128 / 64 / 32, one CTA per SM)
-// instead of two co-resident CTAs with half the ring each.  bn | 0x1000 forces the deep ring, bn | 0x2000 the shallow.
-bool skinny_rule(int M, int N, int K);       // gemm_skinny.cu
-static int deep_mode(int bn) { return (bn & 0x1000) ? 1 : ((bn & 0x2000) ? 0 : -1); }
-static int wants_deep(int M, int N, int bn, int splitk) {
-  static int forced = -2;                                  // RONN_GEMM_RING = deep | shallow overrides the choice
+// instead of two co-resident CTAs with half the ring each.  bn | 0x1000 asks for the deep ring, bn | 0x2000 for the
+// shallow one, RONN_GEMM_RING = deep | shallow for either in every call that does not say.
+static int asked_ring(int bn) {
+  if (bn & 0x3000) return (bn & 0x1000) ? 1 : 0;
+  static int forced = -2;
   if (forced == -2) {
     const char* e = getenv("RONN_GEMM_RING");
     forced = !e ? -1 : (e[0] == 'd' ? 1 : (e[0] == 's' ? 0 : -1));
   }
-  if (forced >= 0) return forced;
+  return forced;
+}
+static int wants_deep(int M, int N, int bn, int splitk) {
   const int tiles = ((N + bn - 1) / bn) * ((M + PG_BM - 1) / PG_BM) * splitk;
   return tiles <= sm_count() ? 1 : 0;
+}
+
+bool skinny_rule(int M, int N, int K);       // gemm_skinny.cu
+
+// The kernel that a call runs: FORM_SKINNY, or the tile width with FORM_DEEP / FORM_SHALLOW (widths of two rings) or
+// FORM_CTA_PAIR.  A width, a pair or a ring that the caller asks for stands.
+constexpr int FORM_SKINNY = 0x8000, FORM_CTA_PAIR = 0x4000, FORM_SHALLOW = 0x2000, FORM_DEEP = 0x1000;
+static int gemm_form(int M, int N, int K, int act, bool residual, bool out_fp32, long ldc, int bn) {
+  if (bn == 0 && skinny_rule(M, N, K)) return FORM_SKINNY;
+  int ring = asked_ring(bn);
+  bool pair = (bn & FORM_CTA_PAIR) != 0;
+  bn &= 0xfff;
+  if (bn == 0 && (M >= 1024 || (M > 256 && pick_bn(M, N) >= 128))) {
+    const TileForm f = pick_form(M, N, K, act, residual, out_fp32);
+    pair = f == FORM_PAIR;
+    bn = f == FORM_64 ? 64 : (f == FORM_128 ? 128 : 256);
+    if (f == FORM_128 && ring < 0) ring = 1;
+  }
+  if (bn == 0) bn = pick_bn(M, N);
+  if (pair) return bn | FORM_CTA_PAIR;
+  if (bn >= 256) return bn;
+  // rows off the 16-byte grid leave through the store-staging area, which only the deep rings carry
+  if (ring < 0) ring = (!out_fp32 && (ldc & 7)) ? 1 : wants_deep(M, N, bn, 1);
+  return bn | (ring ? FORM_DEEP : FORM_SHALLOW);
 }
 
 }  // namespace ronn
@@ -224,8 +250,13 @@ extern "C" int ronn_gemm_skinny(const void* A, const void* W, void* C, const voi
                                 const void* gamma, const void* beta, float eps, int norm, int M, int N, int K, long lda,
                                 long ldw, long ldc, int dtype, int act, int out_fp32, cudaStream_t stream);
 
-// dtype: 0 = bf16, 1 = fp16.  act: 0 none, 1 relu, 2 gelu.  bn: 0 = auto, else 32|64|128|256, or 256 | 0x4000 for CTA pairs (| 0x1000 deep ring,
-// | 0x2000 shallow ring; default picks by tile count).
+// The form that ronn_gemm runs for these arguments (see gemm_form).
+extern "C" int ronn_gemm_form(int M, int N, int K, int act, int residual, int out_fp32, long ldc, int bn) {
+  return gemm_form(M, N, K, act, residual != 0, out_fp32 != 0, ldc, bn);
+}
+
+// dtype: 0 = bf16, 1 = fp16.  act: 0 none, 1 relu, 2 gelu.  bn: 0 = auto, else 32|64|128|256, or 256 | 0x4000 for CTA
+// pairs; | 0x1000 deep ring, | 0x2000 shallow ring.
 // lda/ldw/ldc in elements; K and the leading dimensions must be multiples of 8.
 // Returns 0 on success, negative on configuration errors.
 extern "C" int ronn_gemm(const void* A, const void* W, void* C, const void* bias, const void* residual, int M, int N,
@@ -233,22 +264,11 @@ extern "C" int ronn_gemm(const void* A, const void* W, void* C, const void* bias
                          uint32_t* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   if ((K & 7) || (lda & 7) || (ldw & 7)) return -2;
-  if (bn == 0 && skinny_rule(M, N, K))
+  const int form = gemm_form(M, N, K, act, residual != nullptr, out_fp32 != 0, ldc, bn);
+  if (form == FORM_SKINNY)
     return ronn_gemm_skinny(A, W, C, bias, residual, nullptr, nullptr, 0.f, 0, M, N, K, lda, ldw, ldc, dtype, act, out_fp32, stream);
-  int deep = deep_mode(bn);
-  bool pair = (bn & 0x4000) != 0;
-  bn &= 0xfff;
-  if (bn == 0 && (M >= 1024 || (M > 256 && pick_bn(M, N) >= 128))) {
-    const TileForm f = pick_form(M, N, K, act, residual != nullptr, out_fp32 != 0);
-    pair = f == FORM_PAIR;
-    bn = f == FORM_64 ? 64 : (f == FORM_128 ? 128 : 256);
-    if (f == FORM_128) deep = 1;
-    if (f == FORM_64) deep = 0;
-  }
-  if (bn == 0) bn = pick_bn(M, N);
-  if (deep < 0) deep = wants_deep(M, N, bn, 1);
-  // rows off the 16-byte grid leave through the store-staging area, which only the deep rings carry
-  if (!out_fp32 && (ldc & 7)) deep = 1;
+  const bool pair = (form & FORM_CTA_PAIR) != 0, deep = (form & FORM_DEEP) != 0;
+  bn = form & 0xfff;
   CUtensorMap ma, mb;
   int rc = make_tmap_2d(&ma, A, uint64_t(M), uint64_t(K), uint64_t(lda), PG_BM, 64, 2);
   if (rc) return rc - 20;
@@ -293,7 +313,7 @@ extern "C" int ronn_gemm_splitk(const void* A, const void* W, float* workspace, 
   const int per = (num_kb + splitk - 1) / splitk;
   splitk = (num_kb + per - 1) / per;
   if (splitk_out) *splitk_out = splitk;
-  int deep = deep_mode(bn);
+  int deep = asked_ring(bn);
   bn &= 0xfff;
   if (bn == 0) bn = N >= 128 ? 128 : (N >= 64 ? 64 : 32);
   if (deep < 0) deep = wants_deep(M, N, bn, splitk);
