@@ -166,36 +166,57 @@ int pick_bn(int M, int N) {
   return 32;
 }
 
-// Tile form of a call with many rows (M >= 1024, or fewer with columns enough for 120 tiles of 128: 768 x 4096 x 1024 GELU
-// took 23.5 us on two 128-wide CTAs per SM, 16.0 on one): the cheapest of four by a model in microseconds, fitted to chains inside
-// a CUDA graph (bf16, M 1024 to 8192, N 768 to 4096, K 768 to 4096; it names the fastest form or one within 6 % of it).
-// Every form pays a fixed part (dependency, set-up, first loads, last epilogue) and per wave of tiles the longer of its
-// main loop and its epilogue:
-//   one-CTA 128 x 256   9.0 + waves x max(0.40 per K block, 5.5; 7.0 with residual, 8.0 with GELU)
-//   pair 256 x 256      7.5 + waves x (0.6 + 0.40 per K block + 0.5 with GELU)
-//   one-CTA 128 x 128   5.5 + waves x (0.2 + 0.30 per K block + 0.5 with residual or GELU), one CTA per SM
-//   one-CTA 128 x 64    5.2 + 0.245 per K block while every SM has at most one tile, else 5 + waves x 0.42 per K block, two per SM
-// Measured, pair / 128 x 256 / 128 x 128 (us): 8192 x 3072 x 768 GELU 43.4 / 55.0 / 52.7; 8192 x 768 x 768 residual 18.7 /
-// 22.1 / 18.5; 8192 x 4096 x 1024 GELU 60.1 / 67.9 / 78.6; 4662 x 1024 x 1024 residual 20.8 / 16.5 / 17.0; 4662 x 50257 x
-// 768 (rows off the 16-byte grid) 412 / 627.
-enum TileForm { FORM_64, FORM_128, FORM_256, FORM_PAIR };
-static TileForm pick_form(int M, int N, int K, int act, bool residual, bool out_fp32) {
+// The kernel that a call runs: FORM_SKINNY, or the tile width with FORM_DEEP / FORM_SHALLOW (widths of two rings) or
+// FORM_CTA_PAIR.
+constexpr int FORM_SKINNY = 0x8000, FORM_CTA_PAIR = 0x4000, FORM_SHALLOW = 0x2000, FORM_DEEP = 0x1000;
+
+// What a call costs in each form, in microseconds of a chain inside a CUDA graph:
+//   start + K blocks x block + epilogue + (waves - 1) x max(K blocks x block + gap, epilogue + drain)
+// `start` (dependency, set-up, first loads) and `block` (64 values of K) have one value while every SM has at most one tile
+// and one beyond; the epilogue grows with GELU, a residual, fp32 results and rows off the 16-byte grid, and sets the pace of
+// a wave when it is longer than the main loop.  Fitted to 84 000 timed forms of 12 000 calls: bf16, 1024 to 8192 rows and,
+// where 128-wide tiles fill the chip, 512 to 1000; N 10 to 8193, K 64 to 4096; plain, ReLU, GELU, residual, both, fp32
+// results, odd row lengths.  Mean error of a form 4 to 7 %.  The form it names takes 0.6 % longer than the fastest on average
+// and 8 % less than the rule by tile count (pick_bn); 0.7 % of the calls take more than 5 % longer than under that rule,
+// odd rows of N 1025 to 4097 at K 2048 the worst (28.6 -> 34.7 us).  On 160 calls of 257, 384 and 640 rows, not fitted: none.
+// What it has to weigh, us: 1024 x 64 x 1024 fp32 8.1 at 32 wide, 9.7 at 64 shallow; 1024 x 768 x 2048 12.3 at 64 deep, 14.6
+// shallow; 8192 x 2304 x 64 residual 23.8 on pairs, 34.4 at 64; 8192 x 3072 x 768 GELU 43.4 / 55.0 / 52.7 on pairs / 256 / 128;
+// 4662 x 50257 x 768 (odd rows) 412 / 627 on pairs / 256.
+struct FormCost {
+  int form;
+  float start_one, start_more, block_one, block_more, epilogue, gelu, residual, fp32, ragged, gap, drain;
+};
+static const FormCost form_costs[] = {
+    {32 | FORM_SHALLOW, 2.00f, 3.06f, 0.31f, 0.31f, 1.57f, 0.35f, 0.48f, 0.61f, 0.f, 0.44f, 0.19f},
+    {32 | FORM_DEEP, 3.21f, 3.21f, 0.25f, 0.25f, 0.93f, 0.38f, 0.27f, 0.22f, 0.71f, 0.41f, 0.17f},
+    {64 | FORM_SHALLOW, 2.34f, 3.71f, 0.31f, 0.32f, 1.67f, 0.40f, 0.81f, 1.58f, 0.f, 1.55f, 0.96f},
+    {64 | FORM_DEEP, 3.14f, 3.23f, 0.24f, 0.25f, 1.11f, 0.57f, 0.51f, 0.99f, 0.59f, 0.59f, 0.23f},
+    {128 | FORM_SHALLOW, 2.60f, 7.31f, 0.33f, 0.72f, 2.96f, 1.35f, 0.90f, 1.75f, 0.f, 1.63f, 2.90f},
+    {128 | FORM_DEEP, 4.06f, 4.07f, 0.25f, 0.27f, 1.56f, 1.22f, 1.01f, 2.03f, 1.28f, 1.03f, 1.22f},
+    {256, 4.26f, 3.62f, 0.32f, 0.41f, 3.99f, 2.08f, 2.27f, 4.36f, 2.27f, 0.18f, 2.07f},
+    {256 | FORM_CTA_PAIR, 4.80f, 4.01f, 0.33f, 0.34f, 2.69f, 1.51f, 0.52f, 0.f, 2.18f, 2.27f, 1.74f},
+};
+// ring: 1 deep, 0 shallow, -1 either.  Rows off the 16-byte grid leave through the store-staging area, which the shallow
+// rings do not carry; a tile more than twice as wide as the result would run mostly empty; pairs write 16 bits.
+static int pick_form(int M, int N, int K, int act, bool residual, bool out_fp32, bool ragged, int ring) {
   const int sms = sm_count();
-  const long mt = (M + 127) / 128, mt2 = (M + 255) / 256;
   const float kb = float((K + 63) / 64);
-  auto waves = [](long tiles, int slots) { return float((tiles + slots - 1) / slots); };
-  const bool gelu = act == 2;
-  const long t64 = mt * ((N + 63) / 64);
-  TileForm best = FORM_64;
-  float cost = t64 <= sms ? 5.2f + 0.245f * kb : 5.f + waves(t64, 2 * sms) * 0.42f * kb;
-  auto offer = [&](TileForm f, float c) {
-    if (c < cost) { cost = c; best = f; }
-  };
-  offer(FORM_128, 5.5f + waves(mt * ((N + 127) / 128), sms) * (0.2f + 0.30f * kb + (gelu || residual ? 0.5f : 0.f)));
-  if (N > 128) {
-    const float epi = gelu ? 8.f : (residual || out_fp32 ? 7.f : 5.5f);
-    offer(FORM_256, 9.f + waves(mt * ((N + 255) / 256), sms) * (0.40f * kb > epi ? 0.40f * kb : epi));
-    if (!out_fp32) offer(FORM_PAIR, 7.5f + waves(mt2 * ((N + 255) / 256), sms / 2) * (0.6f + 0.40f * kb + (gelu ? 0.5f : 0.f)));
+  int best = 0;
+  float cost = 1e30f;
+  for (const FormCost& f : form_costs) {
+    const int bn = f.form & 0xfff;
+    const bool pair = (f.form & FORM_CTA_PAIR) != 0, shallow = (f.form & FORM_SHALLOW) != 0;
+    if ((bn > 32 && N <= bn / 2) || (pair && out_fp32)) continue;
+    if (bn < 256 && (ring >= 0 ? shallow == (ring == 1) : shallow && ragged)) continue;
+    const long tiles = long((M + (pair ? 255 : 127)) / (pair ? 256 : 128)) * ((N + bn - 1) / bn);
+    const long slots = pair ? sms / 2 : (shallow ? 2 * sms : sms);
+    const bool one = tiles <= sms;
+    const float epi = f.epilogue + (act == 2 ? f.gelu : 0.f) + (residual ? f.residual : 0.f) + (out_fp32 ? f.fp32 : 0.f) +
+                      (ragged ? f.ragged : 0.f);
+    const float main = kb * (one ? f.block_one : f.block_more);
+    const float wave = main + f.gap > epi + f.drain ? main + f.gap : epi + f.drain;
+    const float t = (one ? f.start_one : f.start_more) + main + epi + float((tiles + slots - 1) / slots - 1) * wave;
+    if (t < cost) { cost = t; best = f.form; }
   }
   return best;
 }
@@ -220,26 +241,18 @@ static int wants_deep(int M, int N, int bn, int splitk) {
 
 bool skinny_rule(int M, int N, int K);       // gemm_skinny.cu
 
-// The kernel that a call runs: FORM_SKINNY, or the tile width with FORM_DEEP / FORM_SHALLOW (widths of two rings) or
-// FORM_CTA_PAIR.  A width, a pair or a ring that the caller asks for stands.
-constexpr int FORM_SKINNY = 0x8000, FORM_CTA_PAIR = 0x4000, FORM_SHALLOW = 0x2000, FORM_DEEP = 0x1000;
+// The form of a call.  A width, a pair or a ring that the caller asks for stands.
 static int gemm_form(int M, int N, int K, int act, bool residual, bool out_fp32, long ldc, int bn) {
   if (bn == 0 && skinny_rule(M, N, K)) return FORM_SKINNY;
-  int ring = asked_ring(bn);
-  bool pair = (bn & FORM_CTA_PAIR) != 0;
+  const int ring = asked_ring(bn);
+  const bool ragged = !out_fp32 && (ldc & 7);
+  if (bn & FORM_CTA_PAIR) return bn & (FORM_CTA_PAIR | 0xfff);
   bn &= 0xfff;
-  if (bn == 0 && (M >= 1024 || (M > 256 && pick_bn(M, N) >= 128))) {
-    const TileForm f = pick_form(M, N, K, act, residual, out_fp32);
-    pair = f == FORM_PAIR;
-    bn = f == FORM_64 ? 64 : (f == FORM_128 ? 128 : 256);
-    if (f == FORM_128 && ring < 0) ring = 1;
-  }
+  if (bn == 0 && (M >= 1024 || (M > 256 && pick_bn(M, N) >= 128)))
+    return pick_form(M, N, K, act, residual, out_fp32, ragged, ring);
   if (bn == 0) bn = pick_bn(M, N);
-  if (pair) return bn | FORM_CTA_PAIR;
   if (bn >= 256) return bn;
-  // rows off the 16-byte grid leave through the store-staging area, which only the deep rings carry
-  if (ring < 0) ring = (!out_fp32 && (ldc & 7)) ? 1 : wants_deep(M, N, bn, 1);
-  return bn | (ring ? FORM_DEEP : FORM_SHALLOW);
+  return bn | ((ring >= 0 ? ring : (ragged ? 1 : wants_deep(M, N, bn, 1))) ? FORM_DEEP : FORM_SHALLOW);
 }
 
 }  // namespace ronn

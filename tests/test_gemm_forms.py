@@ -44,3 +44,59 @@ def test_a_tile_alone_on_its_sm_has_the_deep_ring(M, N, K):
     f = form(M, N, K)
     tiles = -(-M // 128) * -(-N // (f & 0xfff))
     assert f & 0xfff == 64 and tiles <= 148 and f & DEEP
+
+
+_NAMES = {"S": SHALLOW, "D": DEEP, "": 0}
+
+# calls with many rows and the microseconds each form took (one B200, bf16, chains inside a CUDA graph): "res" with a
+# residual, "f32" fp32 results, "rag" an odd row length; S the shallow, D the deep ring
+_MEASURED = [
+    (1024, 10, 64, "plain", "32S:4.3 32D:4.7"),
+    (4096, 10, 128, "f32", "32S:4.7 32D:5.0"),
+    (1024, 64, 1024, "f32", "32S:8.4 32D:7.7 64S:9.5 64D:8.8"),
+    (8192, 32, 256, "gelu", "32S:5.1 32D:5.3"),
+    (4096, 96, 512, "plain", "32S:6.0 32D:6.2 64S:6.4 64D:6.0 128D:7.1"),
+    (1024, 128, 4096, "f32", "32S:22.8 32D:19.3 64S:23.4 64D:20.4 128D:22.8"),
+    (8192, 128, 256, "plain", "32S:6.1 32D:6.4 64S:5.3 64D:5.4 128D:6.5"),
+    (1024, 768, 64, "plain", "32S:4.7 32D:5.3 64S:4.7 64D:4.4 128D:5.7 256:8.1 PAIR:7.4"),
+    (1024, 768, 768, "gelu", "32S:8.8 32D:10.8 64S:8.8 64D:8.1 128D:9.5 256:13.9 PAIR:12.7"),
+    (1024, 768, 2048, "res", "32S:15.3 32D:20.1 64S:14.7 64D:13.0 128D:14.9 256:20.0 PAIR:18.0"),
+    (1536, 768, 768, "gelures", "32S:9.8 32D:11.8 64S:9.1 64D:9.1 128D:10.9 256:16.6 PAIR:13.5"),
+    (1536, 1024, 2048, "plain", "32S:24.5 32D:28.9 64S:15.6 64D:20.4 128D:14.0 256:18.0 PAIR:18.0"),
+    (1536, 2304, 768, "plain", "64S:14.3 64D:14.9 128D:12.5 256:12.3 PAIR:12.2"),
+    (2048, 1024, 4096, "res", "32S:44.6 32D:67.8 64S:27.2 64D:37.1 128D:24.6 256:33.3 PAIR:28.9"),
+    (3000, 1024, 1024, "gelu", "32S:21.1 32D:29.9 64S:16.6 64D:18.0 128D:16.3 256:15.9 PAIR:14.9"),
+    (512, 4096, 1024, "gelu", "64S:11.5 64D:13.9 128D:11.8 256:15.9 PAIR:14.2"),
+    (768, 3072, 256, "plain", "64S:7.4 64D:7.8 128D:7.7 256:10.8 PAIR:8.8"),
+    (1000, 8192, 512, "relu", "64S:18.3 64D:21.7 128D:19.0 256:18.7 PAIR:15.9"),
+    (4096, 1536, 128, "res", "64S:14.9 64D:13.9 128D:13.9 256:18.3 PAIR:13.5"),
+    (8192, 2304, 64, "res", "64S:34.4 64D:31.4 128D:30.3 256:32.7 PAIR:23.8"),
+    (8192, 3072, 768, "gelu", "64S:60.2 64D:77.4 128D:52.5 256:55.7 PAIR:43.3"),
+    (4662, 2304, 4096, "f32", "64S:117.7 64D:149.8 128D:100.1 256:88.3"),
+    (8192, 4096, 2048, "plain", "64S:182.3 64D:261.9 128D:138.5 256:101.4 PAIR:101.7"),
+    (4662, 8193, 128, "rag", "64D:90.7 128D:93.8 256:95.5 PAIR:64.4"),
+    (2048, 769, 512, "rag", "32D:11.9 64D:9.5 128D:9.1 256:13.2 PAIR:12.5"),
+    (8192, 193, 1024, "rag", "32D:22.1 64D:13.9 128D:11.5 256:15.2 PAIR:14.9"),
+    (8192, 8192, 1024, "relu", "64S:189.8 64D:267.6 128D:153.1 256:111.6 PAIR:114.4"),
+]
+
+
+@pytest.mark.parametrize("M,N,K,variant,times", _MEASURED)
+def test_the_chosen_form_is_near_the_fastest(M, N, K, variant, times):
+    us = {}
+    for entry in times.split():
+        name, t = entry.split(":")
+        us[PAIR | 256 if name == "PAIR" else int(name.rstrip("SD")) | _NAMES[name.lstrip("0123456789")]] = float(t)
+    f = form(M, N, K, "gelu" if "gelu" in variant else "relu" if variant == "relu" else "", "res" in variant, variant == "f32",
+             ldc=N if variant == "rag" else None)
+    assert f in us and us[f] <= 1.1 * min(us.values())
+
+
+def test_calls_between_the_rows_of_a_tile():
+    """Every count of rows and columns gives a form that the launcher has, also far outside the measured range."""
+    known = {w | r for w in (32, 64, 128) for r in (DEEP, SHALLOW)} | {256, PAIR | 256, SKINNY}
+    for M in (1, 17, 97, 128, 257, 1023, 1024, 1025, 100000, 2 ** 30):
+        for N in (1, 7, 32, 33, 64, 65, 128, 129, 50257, 2 ** 30):
+            for fp32 in (False, True):
+                f = form(M, N, 8, fp32=fp32, ldc=N)
+                assert f in known and not (fp32 and f & PAIR), (M, N, fp32, hex(f))

@@ -72,3 +72,29 @@ def test_automatic_forms_agree(M, N, Kd):
     y = K.gemm(x, w, bias, res, "gelu")
     K.check_status()
     assert ((y.double() - want).norm() / want.norm()).item() < TOL[torch.bfloat16]
+
+
+# the automatic choice on a chip of 148 SMs, one size and more for every form that it has; every value within its own bound, so
+# that a single lost or misplaced piece of a row shows: the rounding of the result (half a unit in the last place: 2^-8 for
+# the 8-bit significand of bf16) and K products summed in fp32 (K x 2^-23 of the sum of their magnitudes, times 1.13 for the slope of GELU)
+@pytest.mark.parametrize("M,N,Kd,act,resid,fp32,width,ring", [
+    (1024, 16, 64, "", False, False, 32, 0x2000), (1024, 10, 64, "", True, False, 32, 0x1000), (1100, 64, 1000, "", False, True, 32, 0x1000),
+    (8192, 520, 64, "relu", True, False, 64, 0x2000), (1030, 768, 768, "gelu", True, False, 64, 0x1000),
+    (1500, 1000, 2048, "", True, False, 128, 0x1000), (8192, 203, 1024, "gelu", False, False, 128, 0x1000),
+    (1536, 8192, 64, "", False, True, 128, 0x2000), (2048, 2304, 4096, "", False, True, 256, 0),
+    (8190, 776, 768, "gelu", True, False, 256, 0x4000), (4662, 4099, 128, "", False, False, 256, 0x4000)])
+def test_every_form_of_the_automatic_choice(M, N, Kd, act, resid, fp32, width, ring):
+    from ronn_b200 import _native
+    from ronn_b200.ops import kernels as K
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        ldc = N if N % 8 else -(-N // 8) * 8
+        assert _native.cuda().ronn_gemm_form(M, N, Kd, K._ACT[act], int(resid), int(fp32), ldc, 0) == width | ring
+    x, w, bias, res = _operands(M, N, Kd, torch.bfloat16)
+    lin = x.double() @ w.double().t() + bias.double()
+    want = F.relu(lin) if act == "relu" else F.gelu(lin, approximate="tanh") if act == "gelu" else lin
+    want = want + res.double() if resid else want
+    out = torch.full((M + 1, N), 7.0, dtype=torch.float32 if fp32 else torch.bfloat16, device="cuda")
+    K.gemm(x, w, bias, res if resid else None, act, out=out[:M])
+    K.check_status()
+    bound = (2 ** -24 if fp32 else 2 ** -8) * want.abs() + 1.13 * Kd * 2 ** -23 * (x.double().abs() @ w.double().abs().t() + bias.double().abs()) + 2 ** -23 * res.double().abs() + 1e-5
+    assert bool(((out[:M].double() - want).abs() <= bound).all()) and bool((out[M] == 7).all())
