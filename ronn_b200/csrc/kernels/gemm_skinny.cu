@@ -298,40 +298,78 @@ static int launch_skinny(const SkinnyArgs& a, cudaStream_t stream) {
 
 // Two row groups per tile (twice the bytes in flight, half the exchanges) once one group per tile would give every CTA
 // of a full grid several tiles anyway.
-static bool wide_tiles(const SkinnyArgs& a) { return (a.N + 7) / 8 > 4 * device_sm_count(); }
+static bool wide_tiles(int N) { return (N + 7) / 8 > 4 * device_sm_count(); }
 
 template <class T, int NORM>
 static int dispatch_skinny(const SkinnyArgs& a, cudaStream_t stream) {
   const bool one = a.M <= 8;
   if constexpr (NORM != 0) {
     if (!one || a.K > SK_STEP_K) return -2;
-    return wide_tiles(a) ? launch_skinny<T, 1, 2, true, NORM>(a, stream) : launch_skinny<T, 1, 1, true, NORM>(a, stream);
+    return wide_tiles(a.N) ? launch_skinny<T, 1, 2, true, NORM>(a, stream) : launch_skinny<T, 1, 1, true, NORM>(a, stream);
   } else {
-  if (a.K > SK_STEP_K) return one ? launch_skinny<T, 1, 1, false, 0>(a, stream) : launch_skinny<T, 2, 1, false, 0>(a, stream);
-  if (one) return wide_tiles(a) ? launch_skinny<T, 1, 2, true, 0>(a, stream) : launch_skinny<T, 1, 1, true, 0>(a, stream);
-  return wide_tiles(a) ? launch_skinny<T, 2, 2, true, 0>(a, stream) : launch_skinny<T, 2, 1, true, 0>(a, stream);
+    if (a.K > SK_STEP_K) return one ? launch_skinny<T, 1, 1, false, 0>(a, stream) : launch_skinny<T, 2, 1, false, 0>(a, stream);
+    if (one) return wide_tiles(a.N) ? launch_skinny<T, 1, 2, true, 0>(a, stream) : launch_skinny<T, 1, 1, true, 0>(a, stream);
+    return wide_tiles(a.N) ? launch_skinny<T, 2, 2, true, 0>(a, stream) : launch_skinny<T, 2, 1, true, 0>(a, stream);
   }
 }
 
-// Whether the skinny kernel takes a plain projection of this size from the tcgen05 kernel.  Up to 16 rows it reads the
-// weights once and wins everywhere; every further 16 rows read them again.  Measured in chains inside a CUDA graph, bf16,
-// weights from DRAM (us, skinny / tcgen05):
-//   M   N 3072 K 1024   N 1024 K 1024   N 768 K 768   N 1024 K 4096   N 50257 K 1024
-//   1     3.6 / 10.6      2.0 / 7.8      1.9 / 6.7      5.6 / 19.4      19.2 / 30.9
-//  16     4.0 / 11.3      2.3 / 8.0      2.1 / 6.8      6.1 / 19.4      20.4 / 32.4
-//  32     6.1 / 10.4      2.8 / 7.9      2.4 / 6.8      6.9 / 19.4      36.5 / 31.9
-//  48     8.1 / 10.1      4.6 / 8.2      2.5 / 7.0     10.7 / 19.6      53.7 / 31.4
-//  64    10.3 / 8.8       4.8 / 8.1      4.0 / 7.1     11.8 / 19.7
-//  96    14.2 / 9.0       6.6 / 8.4      4.3 / 7.4     17.0 / 19.8
-// The line lies where weights x passes reach 12 Mi values (24 MB).
+// Whether the skinny kernel takes a plain projection of this size from the tcgen05 kernel.
+//
+// Up to 16 rows it reads the weights once and wins (N 10 to 50257, K 64 to 8192), but for 9 to 16 rows against matrices of
+// 64 Mi values and more that the other kernel holds in one wave: 12 x 8192 x 8192 40 / 37 us, 16 x 16384 x 4096 37 / 28.
+// What it still loses there: 8 x 16384 x 8192 63 / 51, 16 x 16384 x 1536 19 / 16, 16 x 8192 x 4096 and 5120 by 8 %.
+//
+// Beyond that every further 16 rows read the weights again, and the two are compared by what they cost, in microseconds of a
+// chain inside a CUDA graph, weights from DRAM (1390 sizes: M 17 to 96, N 10 to 50257, K 64 to 8192, bf16):
+//   skinny   1.1 + waves of CTAs x (0.6 + 0.24 per 8 weight rows of a CTA) + 0.46 per million weights and slice
+//   tcgen05  3.15 + 0.23 per K block + 0.23 per million weights, and when the tiles are more than the SMs
+//            5.6 per further wave of two tiles per SM + 0.36 per K block and wave
+// Where it names the skinny kernel the other is at most 8 % faster; where it names the other, 15 sizes of N 3072 and more and
+// K 512 to 1536 would be 5 to 24 % faster here (40 x 3072 x 1024 7.8 / 9.2, 17 x 50257 x 1024 35 / 43).  By weights and slices alone (a line at 12 Mi values) short K went to the wrong side: 96 x 16384 x 64 19.7 / 5.2 us, 64 x 3072
+// x 1024 10.1 / 7.5, and long K stayed on it: 64 x 1024 x 4096 11.9 / 18.7.
+//   us, skinny / tcgen05   N 3072 K 1024   N 1024 K 1024   N 768 K 768   N 1024 K 4096   N 8192 K 256
+//   M  1                     3.6 / 10.7      2.0 / 7.1      1.9 / 6.1      5.3 / 18.6      3.0 / 5.2
+//     16                     3.8 / 10.1      2.4 / 7.0      2.1 / 6.0      6.2 / 18.5      3.3 / 5.1
+//     32                     6.0 / 9.4       2.8 / 7.0      2.5 / 6.0      7.0 / 18.5      5.5 / 5.0
+//     48                     8.2 / 8.8       4.5 / 7.2      2.5 / 6.1     11.5 / 18.6      7.5 / 5.0
+//     64                    10.1 / 7.5       4.7 / 7.0      4.1 / 6.0     11.9 / 18.7      9.7 / 5.0
+//     96                    14.3 / 7.7       6.6 / 7.0      4.3 / 6.2     16.7 / 18.7     13.8 / 5.0
+int pick_bn(int M, int N);                     // gemm_umma.cu: tile width of the tcgen05 kernel for few rows
 bool skinny_rule(int M, int N, int K) {
-  if (M <= 16) return true;
-  return M <= 96 && long((M + 15) / 16) * N * K <= (12l << 20);
+  if (M <= 8) return true;
+  if (M > 96) return false;
+  const int sms = device_sm_count(), bn = pick_bn(M, N);
+  const int tiles = (N + bn - 1) / bn;
+  const float mega = float(N) * float(K) * 1e-6f;
+  if (M <= 16) return tiles > sms || mega < 67.1f;
+  const int slices = (M + 15) / 16, groups = K <= SK_STEP_K && wide_tiles(N) ? 2 : 1;
+  const int sk_tiles = (N + 8 * groups - 1) / (8 * groups), grid = sk_tiles < 2 * sms ? sk_tiles : 2 * sms;
+  const int waves = (grid * slices + 2 * sms - 1) / (2 * sms), own = (sk_tiles + grid - 1) / grid;
+  // past the register-resident limit a step is 1024 values of K, whole or not
+  const float padded = K <= SK_STEP_K ? 1.f : float((K + SK_STEP_K - 1) / SK_STEP_K * SK_STEP_K) / float(K);
+  const float skinny = 1.1f + float(waves) * (0.6f + 0.24f * float(own * groups)) + 0.46f * float(slices) * mega * padded;
+  const float kb = float((K + 63) / 64);
+  float umma = 3.15f + 0.23f * kb + 0.23f * mega;
+  if (tiles > sms) {
+    const float w = float((tiles + 2 * sms - 1) / (2 * sms));
+    umma += 5.6f * (w - 1.f) + 0.36f * kb * w;
+  }
+  return skinny < umma;
 }
 
 }  // namespace ronn
 
 using namespace ronn;
+
+// Whether a projection whose result a norm reads next is faster as one skinny GEMM followed by the norm kernel than as four
+// K slices on tcgen05 whose reduction applies the norm: where a plain GEMM takes the skinny kernel and its CTAs run as one
+// wave, or up to 16 rows against 8 Mi weights.  Measured, us with the norm, skinny / slices: 16 x 1024 x 4096 8.3 / 10.2, 32 x
+// 1024 x 4096 9.5 / 10.2, 48 x 768 x 2048 7.0 / 8.5, 64 x 512 x 8192 13.1 / 14.1; past one wave 48 x 1024 x 2048 9.3 / 8.3,
+// 80 x 512 x 4096 11.4 / 10.4, 32 x 2048 x 2048 10.7 / 8.8; not skinny at all (few unsliced tiles): 128 x 256 x 2048 13.4 / 9.2.
+extern "C" int ronn_skinny_down_ok(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0 || !skinny_rule(M, N, K)) return 0;
+  return long((M + 15) / 16) * ((N + 7) / 8) <= 2 * device_sm_count() || (M <= 16 && long(N) * K <= (8l << 20));
+}
 
 // out[M,N] = act(norm(A)[M,K] W[N,K]^T + bias) + residual for few rows.  norm: 0 none, 1 LayerNorm, 2 RMSNorm over K
 // (K <= 1024; gamma, and for LayerNorm optionally beta).  dtype 0 bf16, 1 fp16; act 0 none, 1 relu, 2 gelu(tanh).

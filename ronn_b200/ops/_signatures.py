@@ -17,6 +17,7 @@ def declare(lib):
 
     sig("ronn_gemm", [V, V, V, V, V, I, I, I, I, I, I, I, I, I, I, V, V])
     sig("ronn_gemm_form", [I, I, I, I, I, I, L, I])
+    sig("ronn_skinny_down_ok", [I, I, I])
     sig("ronn_gemm_skinny", [V, V, V, V, V, V, V, F, I, I, I, I, L, L, L, I, I, I, V])
     sig("ronn_gemm_splitk", [V, V, V, I, I, I, I, I, I, I, I, V, V, V])
     sig("ronn_splitk_finalize", [V, I, V, V, V, V, V, V, L, I, F, I, I, I, V])

@@ -103,9 +103,8 @@ def norm_gemm_ok(rows: int, k: int) -> bool:
 
 def skinny_down_ok(rows: int, n: int, k: int) -> bool:
     """Whether a long-K projection is faster as one skinny GEMM followed by a norm kernel than as split-K partial sums
-    whose reduction applies the norm (measured, us with the norm: N 1024 K 4096: 16 rows 8.4 / 9.9, 32 rows 9.2 / 10.1,
-    48 rows 13.0 / 10.3; N 768 K 3072: 48 rows 8.1 / 9.7, 64 rows 10.9 / 10.0): up to 8 Mi values of weights x passes."""
-    return -(-rows // 16) * n * k <= 8 << 20
+    whose reduction applies the norm (the native rule, which has the measurements)."""
+    return bool(_native.cuda().ronn_skinny_down_ok(rows, n, k))
 
 
 def norm_gemm(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor], eps: float, norm: str,

@@ -92,6 +92,31 @@ def test_the_chosen_form_is_near_the_fastest(M, N, K, variant, times):
     assert f in us and us[f] <= 1.1 * min(us.values())
 
 
+# few rows: microseconds of the skinny and of the tcgen05 kernel, weights from DRAM, short and long K, on both sides of the line
+@pytest.mark.parametrize("M,N,K,skinny,umma", [
+    (1, 10, 64, 1.4, 3.6), (8, 50257, 1024, 19.3, 43.5), (16, 1024, 4096, 6.2, 18.5), (12, 8192, 8192, 40.0, 37.1),
+    (32, 1024, 1024, 2.8, 7.0), (48, 2304, 768, 6.3, 6.5), (64, 3072, 1024, 10.1, 7.5), (72, 2304, 768, 9.3, 6.4),
+    (64, 8192, 64, 9.1, 3.8), (96, 16384, 64, 19.7, 5.2), (32, 50257, 64, 18.4, 10.3), (56, 512, 8192, 10.7, 33.9),
+    (64, 1024, 4096, 11.9, 18.7), (96, 768, 3072, 10.4, 14.7), (96, 4096, 256, 10.3, 4.7), (32, 1024, 8192, 11.4, 34.0),
+    (17, 3072, 3072, 12.9, 22.6), (96, 2304, 2048, 21.0, 11.1)])
+def test_few_rows_take_the_faster_kernel(M, N, K, skinny, umma):
+    taken = skinny if form(M, N, K) == SKINNY else umma
+    assert taken <= 1.1 * min(skinny, umma)
+
+
+# microseconds with the norm that follows: one skinny launch and a norm kernel, four K slices and a reduction with the norm
+@pytest.mark.parametrize("rows,n,k,one,slices", [
+    (1, 1024, 4096, 6.9, 10.2), (16, 1024, 4096, 8.3, 10.2), (16, 4096, 2048, 10.2, 12.8), (32, 1024, 4096, 9.5, 10.2),
+    (48, 768, 2048, 7.0, 8.5), (64, 512, 8192, 13.1, 14.1), (48, 1024, 2048, 9.3, 8.3), (48, 1024, 4096, 13.5, 10.4),
+    (80, 512, 4096, 11.4, 10.4), (32, 2048, 2048, 10.7, 8.8), (64, 1024, 2048, 10.2, 8.5), (96, 512, 4096, 12.0, 10.5),
+    (128, 256, 2048, 13.4, 9.2), (128, 256, 4096, 21.1, 11.1), (256, 256, 2048, 13.4, 9.2), (512, 512, 2048, 14.0, 10.0)])
+def test_down_projections_take_the_faster_way(rows, n, k, one, slices):
+    from ronn_b200.ops.kernels import skinny_down_ok
+    ok = skinny_down_ok(rows, n, k)
+    assert (one if ok else slices) <= 1.05 * min(one, slices)
+    assert not ok or form(rows, n, k, residual=True) == SKINNY
+
+
 def test_calls_between_the_rows_of_a_tile():
     """Every count of rows and columns gives a form that the launcher has, also far outside the measured range."""
     known = {w | r for w in (32, 64, 128) for r in (DEEP, SHALLOW)} | {256, PAIR | 256, SKINNY}

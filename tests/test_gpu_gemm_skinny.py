@@ -78,3 +78,40 @@ def test_strided_operands_and_refusals(K):
     nan[2, 3] = float("nan")
     y = K.gemm(nan, w)
     assert bool(y[2].isnan().all()) and torch.equal(y[[0, 1, 3, 4]], K.gemm(x, w)[[0, 1, 3, 4]])
+
+
+# four, five and six slices of 16 rows, whatever the automatic choice takes: K in registers and streamed, K off the 32-value piece,
+# two row groups per tile (N past 4736 on 148 SMs), the last slice with one row and whole.  Every value within its own bound:
+# the rounding of the result (2^-24 for fp32, 2^-8 and 2^-11 for bf16 and fp16), K products summed in fp32 (K x 2^-23 of the
+# sum of their magnitudes, times 1.13 for the slope of GELU) and 2^-18 of a GELU's value for its fast exponential
+@pytest.mark.parametrize("M,N,Kd", [(49, 136, 1032), (64, 768, 3072), (65, 131, 2568), (80, 4800, 72), (81, 1000, 512), (96, 7, 8), (96, 768, 3072), (96, 5000, 1024)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("act", ["", "gelu"])
+def test_up_to_six_slices(K, M, N, Kd, dtype, act):
+    from ronn_b200 import _native
+    x, w, bias, res = _operands(M, N, Kd, dtype)
+    lin = x.double() @ w.double().t() + bias.double()
+    ref = F.gelu(lin, approximate="tanh") if act == "gelu" else lin
+    sums = 1.13 * Kd * 2 ** -23 * (x.double().abs() @ w.double().abs().t() + bias.double().abs()) + 2 ** -18 * ref.abs() + 1e-6
+    for out_dtype, r in ((torch.float32, None), (dtype, res)):
+        out = torch.full((M + 1, N), 7.0, dtype=out_dtype, device="cuda")
+        rc = _native.cuda().ronn_gemm_skinny(x.data_ptr(), w.data_ptr(), out.data_ptr(), bias.data_ptr(), K._ptr(r), None, None, 0.0, 0,
+                                             M, N, Kd, Kd, Kd, N, K._DT[dtype], K._ACT[act], int(out_dtype == torch.float32), K._stream())
+        want = ref if r is None else ref + r.double()
+        u = {torch.float32: 2 ** -24, torch.bfloat16: 2 ** -8, torch.float16: 2 ** -11}[out_dtype]
+        assert rc == 0 and bool(((out[:M].double() - want).abs() <= u * want.abs() + sums + 2 ** -23 * res.double().abs()).all())
+        assert bool((out[M] == 7).all())
+
+
+# both sides of the line between the few-rows kernel and the tiles, up to its last row
+@pytest.mark.parametrize("M,N,Kd,skinny", [(48, 2304, 768, True), (64, 2304, 768, False), (96, 768, 3072, True), (97, 768, 3072, False),
+                                           (64, 1024, 4096, True), (64, 8192, 64, False), (16, 8192, 64, True), (32, 768, 768, True)])
+def test_both_sides_of_the_line(K, M, N, Kd, skinny):
+    from ronn_b200 import _native
+    assert (_native.cuda().ronn_gemm_form(M, N, Kd, 0, 1, 0, N, 0) == 0x8000) == skinny
+    x, w, bias, res = _operands(M, N, Kd, torch.bfloat16)
+    ref = x.double() @ w.double().t() + bias.double() + res.double()
+    y = K.gemm(x, w, bias, res)
+    K.check_status()
+    bound = 2 ** -8 * ref.abs() + Kd * 2 ** -23 * (x.double().abs() @ w.double().abs().t()) + 2 ** -22 * (bias.double().abs() + res.double().abs()) + 1e-6
+    assert bool(((y.double() - ref).abs() <= bound).all())
