@@ -128,20 +128,25 @@ def norm_gemm(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor]
     return out
 
 
+_NORM_TYPES = (torch.bfloat16, torch.float16)
+
+
 def _check_norm_operands(x, residual, *params) -> None:
-    """The norm kernels read addresses as rows and parameters of H values of x's type: refuse what is not that."""
-    H = x.shape[-1] if x.dim() else 0
-    if x.dtype not in (torch.bfloat16, torch.float16) or x.device.type != "cuda" or H % 8 or not 0 < H <= 32768:
+    """The norm kernels read addresses as rows and parameters of H values of x's type: refuse what is not that.  In front of
+    every norm launch of an eager session, so it asks for nothing twice (1.6 us of host time)."""
+    shape, dt, dev = x.shape, x.dtype, x.get_device()                    # device index, -1 on the host
+    H = shape[-1] if shape else 0
+    if dt not in _NORM_TYPES or dev < 0 or H % 8 or not 0 < H <= 32768:
         raise OperandError(f"the norm kernel needs 16-bit rows of a multiple of 8 up to 32768 values on a CUDA device, got "
-                           f"{tuple(x.shape)} {x.dtype} on {x.device}")
+                           f"{tuple(shape)} {dt} on device {dev}")
     for p in params:
-        if p is not None and (p.dtype != x.dtype or p.device != x.device or p.numel() != H or not p.is_contiguous()
+        if p is not None and (p.dtype is not dt or p.get_device() != dev or p.numel() != H or not p.is_contiguous()
                               or p.data_ptr() % 16):
-            raise OperandError(f"norm parameters must be {H} values of {x.dtype} on {x.device}, contiguous from a 16-byte "
-                               f"boundary, got {tuple(p.shape)} {p.dtype} on {p.device}")
-    if residual is not None and (residual.dtype != x.dtype or residual.device != x.device or residual.numel() != x.numel()):
+            raise OperandError(f"norm parameters must be {H} values of {dt} on device {dev}, contiguous from a 16-byte "
+                               f"boundary, got {tuple(p.shape)} {p.dtype} on device {p.get_device()}")
+    if residual is not None and (residual.dtype is not dt or residual.get_device() != dev or residual.numel() != x.numel()):
         raise OperandError(f"the norm's residual must match its input, got {tuple(residual.shape)} {residual.dtype} on "
-                           f"{residual.device}")
+                           f"device {residual.get_device()}")
 
 
 def _norm(x, gamma, beta, residual, eps, rms, sum_out):
