@@ -778,15 +778,24 @@ static void bitlinear_plan(int M, int N, int K, bool may_slice, int& bn, int& S)
 constexpr int BL_EXPAND_ROWS = 1024;
 static bool bitlinear_expands(int M, int K) { return M >= BL_EXPAND_ROWS && (K & 63) == 0; }
 
-// Bytes of scratch memory a call of this shape wants: for the expanded weights of a call with many rows (one byte per
-// weight), or for its K slices (at most one CTA per SM is sliced, so never above 148 x 64 KB); 0: none.
-extern "C" long ronn_bitlinear_workspace_bytes(int M, int N, int K) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (bitlinear_expands(M, K)) return long(N) * K;
+static long bitlinear_slice_bytes(int M, int N, int K) {
   int bn, S;
   bitlinear_plan(M, N, K, true, bn, S);
-  if (S == 1) return 0;
-  return long((M + 127) / 128) * ((N + bn - 1) / bn) * S * bn * 512;
+  return S == 1 ? 0 : long((M + 127) / 128) * ((N + bn - 1) / bn) * S * bn * 512;
+}
+
+// Bytes of scratch memory a ronn_bitlinear call of this shape wants: for the expanded weights of a call with many rows (one
+// byte per weight), or for its K slices (at most one CTA per SM is sliced, so never above 148 x 64 KB); 0: none.  Enough for
+// the slices in either case: weights off the 16-byte grid are not expanded.
+extern "C" long ronn_bitlinear_workspace_bytes(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const long slices = bitlinear_slice_bytes(M, N, K), expanded = bitlinear_expands(M, K) ? long(N) * K : 0;
+  return slices > expanded ? slices : expanded;
+}
+
+// The same for ronn_bitlinear_to_slot, which never expands: its slices only.
+extern "C" long ronn_bitlinear_slot_workspace_bytes(int M, int N, int K) {
+  return M <= 0 || N <= 0 || K <= 0 ? 0 : bitlinear_slice_bytes(M, N, K);
 }
 
 // x: [rows, 2 F] (gate | up), dtype 0 bf16 / 1 fp16 -> q int8 [rows, F], scale fp32 [rows].
@@ -803,8 +812,8 @@ extern "C" int ronn_swiglu_quant_int8(const void* x, void* q, float* scale, long
 }
 
 // xq: int8 [M, K] (row stride ldx bytes); w_packed: [N, K/4]; x_scale: fp32 [M]; out: [M, N] in `dtype` (0 bf16, 1 fp16).
-// K % 16 == 0 and ldx % 16 == 0.  workspace: null, or ronn_bitlinear_workspace_bytes(M, N, K) bytes (16-byte aligned)
-// that no other call in flight uses; without it the K range is not sliced.
+// K % 16 == 0 and ldx % 16 == 0.  workspace: null, or as many bytes as the entry point's query says (16-byte aligned)
+// that no other call in flight uses; without it the K range is not sliced and the weights are not expanded.
 static int bitlinear_impl(const void* xq, const void* w_packed, const float* x_scale, float w_scale, const void* bias,
                           void* out, int M, int N, int K, int ldx, int dtype, const int* slot_state, long slot_stride,
                           void* workspace, uint32_t* status, cudaStream_t stream) {
@@ -815,8 +824,7 @@ static int bitlinear_impl(const void* xq, const void* w_packed, const float* x_s
     return dtype == 0 ? launch_bitlinear_pair<__nv_bfloat16>(xq, w_packed, x_scale, w_scale, bias, out, M, N, K, ldx, status, stream, workspace)
                       : launch_bitlinear_pair<__half>(xq, w_packed, x_scale, w_scale, bias, out, M, N, K, ldx, status, stream, workspace);
   int bn, S;
-  // scratch that was sized for expanded weights is not used for K slices
-  bitlinear_plan(M, N, K, workspace != nullptr && !bitlinear_expands(M, K), bn, S);
+  bitlinear_plan(M, N, K, workspace != nullptr, bn, S);
   CUtensorMap mx;
   int rc = make_tmap_2d(&mx, xq, uint64_t(M), uint64_t(K), uint64_t(ldx), 128, 128, 1);
   if (rc) return rc - 20;

@@ -50,13 +50,15 @@ def swiglu_quant_int8(x: torch.Tensor):
 _WS_BYTES = {}
 
 
-def slice_workspace(M: int, n: int, k: int, device) -> Optional[torch.Tensor]:
-    """Scratch memory for the K slices of a skinny BitLinear call (None when the shape is not sliced).  A fresh tensor per
-    call: calls on concurrent streams must not share it, and inside a CUDA-graph capture it comes from the graph's pool."""
-    key = (M, n, k)
+def slice_workspace(M: int, n: int, k: int, device, slot: bool = False) -> Optional[torch.Tensor]:
+    """Scratch memory of a BitLinear call: K slices of a skinny one, expanded weights of one with many rows (None when the
+    shape wants none); ``slot``: of ``ronn_bitlinear_to_slot``, which only slices.  A fresh tensor per call: calls on
+    concurrent streams must not share it, and inside a CUDA-graph capture it comes from the graph's pool."""
+    key = (M, n, k, slot)
     nbytes = _WS_BYTES.get(key)
     if nbytes is None:
-        nbytes = int(_native.cuda().ronn_bitlinear_workspace_bytes(M, n, k))
+        lib = _native.cuda()
+        nbytes = int((lib.ronn_bitlinear_slot_workspace_bytes if slot else lib.ronn_bitlinear_workspace_bytes)(M, n, k))
         _WS_BYTES[key] = nbytes
     return torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes else None
 

@@ -450,7 +450,7 @@ class FusedComm(TPComm):
         stream = torch.cuda.current_stream().cuda_stream
         status = K.status_word(q.device).data_ptr()
         from ..ops.bitnet import slice_workspace
-        ws = slice_workspace(M, n, k, q.device)
+        ws = slice_workspace(M, n, k, q.device, slot=True)
         _bcheck(lib.ronn_bitlinear_to_slot(q.data_ptr(), w_packed.data_ptr(), x_scale.data_ptr(), float(w_scale),
                                            self._part_ptrs[self.rank], self._state.data_ptr(), self.part_stride,
                                            None if ws is None else ws.data_ptr(), M, n, k,

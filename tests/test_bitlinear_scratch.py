@@ -1,0 +1,51 @@
+"""Scratch memory and launch plan of BitLinear calls: asked of the native rules on the host, and the slot form on the device."""
+import pytest
+import torch
+
+from ronn_b200 import _native
+
+
+def _bytes(M, N, K, slot=False):
+    lib = _native.cuda()
+    return (lib.ronn_bitlinear_slot_workspace_bytes if slot else lib.ronn_bitlinear_workspace_bytes)(M, N, K)
+
+
+# one byte per weight from 1024 rows on, K a multiple of 64; never less than the slices that the same call falls back to
+@pytest.mark.parametrize("M,N,K", [(1024, 256, 2560), (1024, 2560, 6912), (8192, 7680, 2560), (1024, 8, 128), (2048, 40, 64)])
+def test_many_rows_expand(M, N, K):
+    assert _bytes(M, N, K) == max(N * K, _bytes(M, N, K, slot=True))
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 2560, 6912), (1023, 256, 2560), (1, 640, 2560), (1100, 136, 48)])
+def test_few_rows_and_other_k_only_slice(M, N, K):
+    assert _bytes(M, N, K) == _bytes(M, N, K, slot=True)
+
+
+def test_the_slot_form_takes_no_scratch_for_expanded_weights():
+    """It never expands: whole wide outputs take none, narrow ones their slices, the same at 1024 rows as just below."""
+    assert _bytes(1024, 2560, 6912, slot=True) == 0 and _bytes(8192, 13824, 2560, slot=True) == 0
+    for N, K in ((256, 2560), (512, 6912), (1024, 6912)):
+        assert 0 < _bytes(1024, N, K, slot=True) == _bytes(1023, N, K, slot=True) <= 148 * 64 * 1024
+
+
+# the result lands in the slot that the state's parity names, with and without slices; exact sums, so one rounding
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(1024, 256, 2560), (1030, 512, 320), (1024, 1024, 6912), (1024, 2560, 640), (96, 640, 2560)])
+@pytest.mark.parametrize("parity", [0, 1])
+def test_slot_form(M, N, K, parity):
+    from ronn_b200.ops import bitnet as B
+    from ronn_b200.ops import kernels as Kn
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    q = torch.randint(-127, 128, (M, K), generator=g, device="cuda", dtype=torch.int8)
+    w = torch.randint(-1, 2, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    s = torch.rand(M, generator=g, device="cuda") * 0.01 + 0.001
+    packed = B.ternary_pack(w)
+    slots = torch.full((2, M, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    state = torch.tensor([4 + parity], dtype=torch.int32, device="cuda")
+    ws = B.slice_workspace(M, N, K, q.device, slot=True)
+    rc = _native.cuda().ronn_bitlinear_to_slot(q.data_ptr(), packed.data_ptr(), s.data_ptr(), 0.043, slots.data_ptr(), state.data_ptr(),
+                                               M * N * 2, None if ws is None else ws.data_ptr(), M, N, K, K, 0,
+                                               Kn.status_word(q.device).data_ptr(), Kn._stream())
+    Kn.check_status()
+    want = ((q.double() @ w.double().t()).float() * (s * torch.tensor(0.043, device="cuda"))[:, None]).bfloat16()
+    assert rc == 0 and torch.equal(slots[parity], want) and bool((slots[1 - parity] == 7).all())
