@@ -562,7 +562,7 @@ bitlinear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // rows) and the expander warps set the pace.  There the packed matrix is expanded once into int8 scratch, 1.25 bytes of
 // traffic per weight, and the product runs as a dense int8 GEMM on CTA pairs.  Same integers, same scaling: same results.
 // 8192 rows, us before / after: N 7680 K 2560 347 / 120, N 13824 K 2560 622 / 215, N 2560 K 6912 256 / 113; 1024 rows:
-// 54 / 29, 81 / 42, 58 / 32.
+// 54 / 29, 81 / 42, 58 / 32.  Narrow outputs and short K stay with the kernel above (bitlinear_expands).
 __global__ void ternary_expand_kernel(const uint4* __restrict__ packed, int4* __restrict__ out, long n16) {
   pdl_wait();                                    // the scratch may belong to the previous kernel of the stream until it ends
   pdl_trigger();
@@ -742,11 +742,13 @@ extern "C" int ronn_norm_quant_int8(const void* x, const void* gamma, void* q, f
 // MMA issuer's loop: every MMA streams its 128 x 32-byte A operand from shared memory, ~70 cycles, four per block,
 // plus ~220 cycles of barrier traffic; wide tiles add expansion time).  Slicing K costs 1.5 us (cluster barrier and
 // an L2 round trip on data other SMs have just written) plus 0.4 us per MB of partial tiles.  The grid runs in waves
-// of one CTA per SM.
-static void bitlinear_plan(int M, int N, int K, bool may_slice, int& bn, int& S) {
+// of one CTA per SM.  Returns the estimate with what a wave of many rows adds (1.4 us of epilogue each, see
+// bitlinear_expands).
+static float bitlinear_plan(int M, int N, int K, bool may_slice, int& bn, int& S) {
   const int mt = (M + 127) / 128, total_kb = (K + 127) / 128, sms = device_sm_count();
   bn = 128;
   S = 1;
+  int best_waves = 1;
   float best = 1e30f;
   const int bns[3] = {128, 64, 32};
   const float per_kb[3] = {0.476f, 0.364f, 0.324f};
@@ -760,7 +762,7 @@ static void bitlinear_plan(int M, int N, int K, bool may_slice, int& bn, int& S)
       const int waves = (ctas + sms - 1) / sms;
       const float part_mb = float(ctas) * float(bns[i]) * 512.f / 1048576.f;
       const float t = float(waves) * (2.3f + per_kb[i] * float(per)) + (s > 1 ? 1.5f + 0.4f * part_mb : 0.f);
-      if (t < best) { best = t; bn = bns[i]; S = s; }
+      if (t < best) { best = t; best_waves = waves; bn = bns[i]; S = s; }
     }
   if (const char* e = getenv("RONN_BITLINEAR_TILE")) {       // "bn,slices" override for experiments
     int b = 0, s = 0;
@@ -770,13 +772,26 @@ static void bitlinear_plan(int M, int N, int K, bool may_slice, int& bn, int& S)
       if (s <= total_kb && (total_kb + per - 1) / per == s && (s == 1 || mt * ((N + b - 1) / b) * s <= sms)) { bn = b; S = s; }
     }
   }
+  return 1.f + best + 1.4f * float(best_waves);
 }
 
-// Whether the weights are worth expanding once for the whole call: from BL_EXPAND_ROWS rows on (about twice as fast there;
-// at 512 rows the tiles of the other kernel still fit two waves), when the packed rows are whole 16-byte pieces (K a
-// multiple of 64).
+// Whether the weights are expanded once for the whole call: from BL_EXPAND_ROWS rows on, when the packed rows are whole
+// 16-byte pieces (K a multiple of 64) and the expansion (6.9 us and 0.41 per million weights) with a dense product on CTA
+// pairs costs less than the kernel that expands in every row tile.  Narrow outputs and short K do not repay it: by rows alone
+// 1024 x 64 x 6912 took 24.4 us instead of 7.9, 1100 x 256 x 64 9.0 instead of 3.5; wide ones do: 8192 x 2560 x 2560 51.6 / 119,
+// 1024 x 2560 x 6912 31.5 / 57.2.  Of 417 calls measured (1024 to 8192 rows, N 8 to 13824, K 64 to 6912) it names the faster
+// way or one within 6 %.
 constexpr int BL_EXPAND_ROWS = 1024;
-static bool bitlinear_expands(int M, int K) { return M >= BL_EXPAND_ROWS && (K & 63) == 0; }
+static bool bitlinear_expands(int M, int N, int K) {
+  if (M < BL_EXPAND_ROWS || (K & 63) != 0) return false;
+  int bn, S;
+  const float tiles_us = bitlinear_plan(M, N, K, true, bn, S);
+  const int pairs = device_sm_count() / 2;
+  const long tiles = long((M + 255) / 256) * ((N + 255) / 256);
+  const float main = 1.75f + 0.30f * float((K + 127) / 128);
+  const float pair_us = 6.9f + 0.41e-6f * float(N) * float(K) + main + float((tiles + pairs - 1) / pairs - 1) * (main > 3.6f ? main : 3.6f);
+  return pair_us < tiles_us;
+}
 
 static long bitlinear_slice_bytes(int M, int N, int K) {
   int bn, S;
@@ -789,7 +804,7 @@ static long bitlinear_slice_bytes(int M, int N, int K) {
 // the slices in either case: weights off the 16-byte grid are not expanded.
 extern "C" long ronn_bitlinear_workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const long slices = bitlinear_slice_bytes(M, N, K), expanded = bitlinear_expands(M, K) ? long(N) * K : 0;
+  const long slices = bitlinear_slice_bytes(M, N, K), expanded = bitlinear_expands(M, N, K) ? long(N) * K : 0;
   return slices > expanded ? slices : expanded;
 }
 
@@ -820,7 +835,7 @@ static int bitlinear_impl(const void* xq, const void* w_packed, const float* x_s
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   if ((K & 15) || (ldx & 15)) return -2;
   if (reinterpret_cast<uintptr_t>(workspace) & 15) return -2;
-  if (workspace != nullptr && slot_state == nullptr && bitlinear_expands(M, K) && (reinterpret_cast<uintptr_t>(w_packed) & 15) == 0)
+  if (workspace != nullptr && slot_state == nullptr && bitlinear_expands(M, N, K) && (reinterpret_cast<uintptr_t>(w_packed) & 15) == 0)
     return dtype == 0 ? launch_bitlinear_pair<__nv_bfloat16>(xq, w_packed, x_scale, w_scale, bias, out, M, N, K, ldx, status, stream, workspace)
                       : launch_bitlinear_pair<__half>(xq, w_packed, x_scale, w_scale, bias, out, M, N, K, ldx, status, stream, workspace);
   int bn, S;
