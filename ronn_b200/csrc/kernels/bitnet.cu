@@ -736,6 +736,12 @@ extern "C" int ronn_norm_quant_int8(const void* x, const void* gamma, void* q, f
   return err == cudaSuccess ? 0 : -100;
 }
 
+// RONN_BITLINEAR_TILE = "bn,slices": the tile width and K slices that an experiment asks for, wherever they fit.
+static bool bitlinear_asked_tile(int& bn, int& S) {
+  const char* e = getenv("RONN_BITLINEAR_TILE");
+  return e && sscanf(e, "%d,%d", &bn, &S) == 2 && (bn == 32 || bn == 64 || bn == 128) && S >= 1 && S <= 8 && bn / S >= 8 && (S & (S - 1)) == 0;
+}
+
 // Tile width and number of K slices: the pair with the lowest estimated time, from a model fitted to measurements
 // (128 x 2560..13824 x 864..6912 in a CUDA graph).  A CTA costs a fixed part (launch, barrier and TMEM set-up, first
 // loads from DRAM: 2.3 us) and 0.32 / 0.36 / 0.48 us per 128-deep K block of its slice for 32 / 64 / 128 columns (the
@@ -764,13 +770,10 @@ static float bitlinear_plan(int M, int N, int K, bool may_slice, int& bn, int& S
       const float t = float(waves) * (2.3f + per_kb[i] * float(per)) + (s > 1 ? 1.5f + 0.4f * part_mb : 0.f);
       if (t < best) { best = t; best_waves = waves; bn = bns[i]; S = s; }
     }
-  if (const char* e = getenv("RONN_BITLINEAR_TILE")) {       // "bn,slices" override for experiments
-    int b = 0, s = 0;
-    if (sscanf(e, "%d,%d", &b, &s) == 2 && (b == 32 || b == 64 || b == 128) && s >= 1 && s <= 8 && b / s >= 8 &&
-        (s & (s - 1)) == 0 && (may_slice || s == 1)) {
-      const int per = (total_kb + s - 1) / s;
-      if (s <= total_kb && (total_kb + per - 1) / per == s && (s == 1 || mt * ((N + b - 1) / b) * s <= sms)) { bn = b; S = s; }
-    }
+  int b = 0, s = 0;
+  if (bitlinear_asked_tile(b, s) && (may_slice || s == 1)) {
+    const int per = (total_kb + s - 1) / s;
+    if (s <= total_kb && (total_kb + per - 1) / per == s && (s == 1 || mt * ((N + b - 1) / b) * s <= sms)) { bn = b; S = s; }
   }
   return 1.f + best + 1.4f * float(best_waves);
 }
@@ -783,8 +786,8 @@ static float bitlinear_plan(int M, int N, int K, bool may_slice, int& bn, int& S
 // way or one within 6 %.
 constexpr int BL_EXPAND_ROWS = 1024;
 static bool bitlinear_expands(int M, int N, int K) {
-  if (M < BL_EXPAND_ROWS || (K & 63) != 0) return false;
   int bn, S;
+  if (M < BL_EXPAND_ROWS || (K & 63) != 0 || bitlinear_asked_tile(bn, S)) return false;      // an asked-for tile stands
   const float tiles_us = bitlinear_plan(M, N, K, true, bn, S);
   const int pairs = device_sm_count() / 2;
   const long tiles = long((M + 255) / 256) * ((N + 255) / 256);

@@ -1,6 +1,7 @@
 """Launch wrappers of the BitNet device kernels (activation quantisation, ternary x int8 BitLinear, packing)."""
 from __future__ import annotations
 
+import os
 from typing import Optional
 
 import torch
@@ -54,7 +55,7 @@ def slice_workspace(M: int, n: int, k: int, device, slot: bool = False) -> Optio
     """Scratch memory of a BitLinear call: K slices of a skinny one, expanded weights of one with many rows (None when the
     shape wants none); ``slot``: of ``ronn_bitlinear_to_slot``, which only slices.  A fresh tensor per call: calls on
     concurrent streams must not share it, and inside a CUDA-graph capture it comes from the graph's pool."""
-    key = (M, n, k, slot)
+    key = (M, n, k, slot, os.environ.get("RONN_BITLINEAR_TILE"))       # the native plan reads it in every call
     nbytes = _WS_BYTES.get(key)
     if nbytes is None:
         lib = _native.cuda()

@@ -42,6 +42,23 @@ def test_the_slot_form_takes_no_scratch_for_expanded_weights():
         assert 0 < _bytes(1024, N, K, slot=True) == _bytes(1023, N, K, slot=True) <= 148 * 64 * 1024
 
 
+# "bn,slices" as asked for, also from 1024 rows on, where it switches the expansion off; what does not fit or is no tile leaves
+# the plan alone
+@pytest.mark.parametrize("tile,scratch", [("64,2", 8 * 4 * 2 * 64 * 512), ("128,4", 8 * 2 * 4 * 128 * 512), ("32,1", 0), ("48,1", None), ("128", None)])
+def test_an_asked_for_tile_stands(tile, scratch, monkeypatch):
+    from ronn_b200.ops import bitnet as B
+    plain = _bytes(1024, 256, 2560)
+    assert _expands(1024, 2560, 2560)
+    monkeypatch.setenv("RONN_BITLINEAR_TILE", tile)
+    assert _bytes(1024, 256, 2560) == (plain if scratch is None else scratch)
+    assert _expands(1024, 2560, 2560) == (scratch is None)
+    ws = B.slice_workspace(1024, 256, 2560, "cpu")
+    assert (0 if ws is None else ws.numel()) == _bytes(1024, 256, 2560)
+    monkeypatch.delenv("RONN_BITLINEAR_TILE")                # the size kept for the shape is not the other plan's
+    ws = B.slice_workspace(1024, 256, 2560, "cpu")
+    assert (0 if ws is None else ws.numel()) == plain
+
+
 # expanded weights: rows past a tile and past its first half, columns cut inside a box, K of one and several blocks and cut inside
 # one, rows of the result on and off the 16-byte grid; exact sums, so one rounding
 @pytest.mark.gpu
@@ -82,3 +99,18 @@ def test_slot_form(M, N, K, parity):
     Kn.check_status()
     want = ((q.double() @ w.double().t()).float() * (s * torch.tensor(0.043, device="cuda"))[:, None]).bfloat16()
     assert rc == 0 and torch.equal(slots[parity], want) and bool((slots[1 - parity] == 7).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile", ["64,2", "128,1", "32,4"])
+def test_an_asked_for_tile_computes_the_same(tile, monkeypatch):
+    from ronn_b200.ops import bitnet as B
+    from ronn_b200.ops import kernels as Kn
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q = torch.randint(-127, 128, (1100, 2560), generator=g, device="cuda", dtype=torch.int8)
+    packed = B.ternary_pack(torch.randint(-1, 2, (264, 2560), generator=g, device="cuda", dtype=torch.int8))
+    s = torch.rand(1100, generator=g, device="cuda") * 0.01 + 0.001
+    plain = B.bitlinear_q(q, s, packed, 0.043, None, 264, 2560, torch.bfloat16)
+    monkeypatch.setenv("RONN_BITLINEAR_TILE", tile)
+    assert torch.equal(B.bitlinear_q(q, s, packed, 0.043, None, 264, 2560, torch.bfloat16), plain)
+    Kn.check_status()
