@@ -318,6 +318,8 @@ static int dispatch_skinny(const SkinnyArgs& a, cudaStream_t stream) {
 // Up to 16 rows it reads the weights once and wins (N 10 to 50257, K 64 to 8192), but for 9 to 16 rows against matrices of
 // 64 Mi values and more that the other kernel holds in one wave: 12 x 8192 x 8192 40 / 37 us, 16 x 16384 x 4096 37 / 28.
 // What it still loses there: 8 x 16384 x 8192 63 / 51, 16 x 16384 x 1536 19 / 16, 16 x 8192 x 4096 and 5120 by 8 %.
+// K of up to 128 gives one or two of the 8 warps weights to read: the vocabulary of a very narrow model, behind its norm kernel,
+// is left to tcgen05 (1 to 8 x 50257 x 64 11.2 / 8.7 with the norm, x 32000 x 128 8.8 / 8.1; x 16384 x 64 stays, 5.6 / 7.0).
 //
 // Beyond that every further 16 rows read the weights again, and the two are compared by what they cost, in microseconds of a
 // chain inside a CUDA graph, weights from DRAM (1390 sizes: M 17 to 96, N 10 to 50257, K 64 to 8192, bf16):
@@ -336,8 +338,8 @@ static int dispatch_skinny(const SkinnyArgs& a, cudaStream_t stream) {
 //     96                    14.3 / 7.7       6.6 / 7.0      4.3 / 6.2     16.7 / 18.7     13.8 / 5.0
 int pick_bn(int M, int N);                     // gemm_umma.cu: tile width of the tcgen05 kernel for few rows
 bool skinny_rule(int M, int N, int K) {
+  if (M > 96 || (K <= 128 && N > 24576)) return false;
   if (M <= 8) return true;
-  if (M > 96) return false;
   const int sms = device_sm_count(), bn = pick_bn(M, N);
   const int tiles = (N + bn - 1) / bn;
   const float mega = float(N) * float(K) * 1e-6f;

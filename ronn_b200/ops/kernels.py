@@ -96,9 +96,11 @@ def gemm(a: torch.Tensor, w_nk: torch.Tensor, bias: Optional[torch.Tensor] = Non
     return out
 
 
-def norm_gemm_ok(rows: int, k: int) -> bool:
-    """Sizes ``norm_gemm`` takes: few rows, a row short enough to stay in the registers of one CTA."""
-    return 0 < rows <= 8 and k <= 1024 and k % 8 == 0
+def norm_gemm_ok(rows: int, k: int, n: int = 0) -> bool:
+    """Sizes ``norm_gemm`` takes: few rows, a row short enough to stay in the registers of one CTA; with ``n`` outputs also
+    whether it is the faster way (a norm kernel and the tcgen05 GEMM read a wide matrix of very short rows sooner: 1 x 50257 x
+    64 8.7 against 11.4 us, 1 x 32000 x 128 8.1 against 8.6, 1 x 50257 x 256 13.9 against 12.8)."""
+    return 0 < rows <= 8 and k <= 1024 and k % 8 == 0 and not (k <= 128 and n > 24576)
 
 
 def skinny_down_ok(rows: int, n: int, k: int) -> bool:

@@ -362,7 +362,7 @@ class DecoderRunner:
         else:
             if not decode:
                 x = ops.gather_rows(x, b["sample_index_clamped"])
-            if ops.name == "kernels" and self.tp == 1 and self._norm_gemm_ok(x.shape[0], a.hidden):
+            if ops.name == "kernels" and self.tp == 1 and self._norm_gemm_ok(x.shape[0], a.hidden, self.lm_head.shape[0]):
                 logits = ops.norm_gemm(x, self.lnf, a.norm, a.eps, self.lm_head, logits=True)
             else:
                 x = self._norm(x, self.lnf)

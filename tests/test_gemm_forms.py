@@ -104,6 +104,18 @@ def test_few_rows_take_the_faster_kernel(M, N, K, skinny, umma):
     assert taken <= 1.1 * min(skinny, umma)
 
 
+# the vocabulary of very narrow models: microseconds with the norm in front, fused into the few-rows kernel or on its own with
+# the tcgen05 kernel
+@pytest.mark.parametrize("M,N,K,fused,apart", [(1, 50257, 64, 11.4, 8.7), (8, 50257, 128, 12.2, 10.7), (4, 32000, 64, 7.6, 6.9),
+                                               (8, 32000, 128, 8.7, 8.1), (1, 16384, 64, 5.4, 7.0), (8, 16384, 128, 5.7, 7.4), (4, 50257, 256, 12.8, 14.1),
+                                               (8, 50257, 1024, 20.0, 44.0)])
+def test_logits_of_a_few_rows(M, N, K, fused, apart):
+    from ronn_b200.ops.kernels import norm_gemm_ok
+    ok = norm_gemm_ok(M, K, N)
+    assert (fused if ok else apart) == min(fused, apart) and (form(M, N, K) == SKINNY) == ok
+    assert norm_gemm_ok(M, K)                                # the kernel takes the size either way
+
+
 # microseconds with the norm that follows: one skinny launch and a norm kernel, four K slices and a reduction with the norm
 @pytest.mark.parametrize("rows,n,k,one,slices", [
     (1, 1024, 4096, 6.9, 10.2), (16, 1024, 4096, 8.3, 10.2), (16, 4096, 2048, 10.2, 12.8), (32, 1024, 4096, 9.5, 10.2),
