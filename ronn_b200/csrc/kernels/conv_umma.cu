@@ -330,8 +330,10 @@ static int launch_conv(const void* x, const CUtensorMap& mw, const ConvShape& cs
 // tap for 128 output positions (padding and the positions past the last image arrive as zeros), so the persistent GEMM
 // main loop runs it like a dense A.  The software gather spends eight address computations and cp.async per thread and K
 // block and was bound by their issue: ResNet-18, one B200, fp16 batch 1 267 -> 176 us, batch 32 698 -> 487 us, bf16 batch
-// 117 1919 -> 1062 us; its 3x3 layers at batch 117 now run at 470 to 775 TFLOP/s.  TAP16: 16 input channels (the space-to-depth stem); a K block of 64 is four taps,
-// each a tile of 128 rows x 32 bytes.
+// 117 1919 -> 1062 us; its 3x3 layers at batch 117 now run at 470 to 775 TFLOP/s.
+// TAP16: 16 input channels and a multiple of four taps (filters over space-to-depth inputs, patches); a K block of 64 is four
+// taps, each a tile of 128 rows x 32 bytes.  us, gather / this: 4 x 4 over 32 x 112 x 112 -> 64 channels 95.9 / 39.1, over 32 x 56
+// x 56 -> 128 49.3 / 20.9, 4 x 4 / 4 over 32 x 56 x 56 -> 256 13.3 / 7.4, over one 56 x 56 -> 64 9.2 / 5.8.
 template <int BN, class T, bool TAP16>
 struct ConvProblem {
   // results leave in 64-byte runs also from the 64-wide tiles, which gave a ring stage for it: the stem at batch 117 (188 MB of
@@ -421,6 +423,13 @@ conv_im2col_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   gemm_persistent<BN, STAGES, 0, ConvProblem<BN, T, TAP16>, KA>(dyn_smem, prob, 64, idesc, status);
 }
 
+// CTAs of an im2col form that one SM holds: by its shared memory (two rings in 228 KB) and TMEM columns
+template <int BN, int STAGES, int KA>
+constexpr int im2col_per_sm() {
+  using L = PGemmSmem<BN, STAGES, true, KA>;
+  return L::DYN_SMEM <= 112 * 1024 && L::TMEM_COLS <= 256 ? 2 : 1;
+}
+
 template <int BN, int STAGES, int KA, class T, bool TAP16>
 static int launch_im2col(const CUtensorMap& ma, const CUtensorMap& mw, const ConvShape& cs, const DenseEpilogue& e, int is_bf16,
                          uint32_t* status, cudaStream_t stream) {
@@ -431,7 +440,7 @@ static int launch_im2col(const CUtensorMap& ma, const CUtensorMap& mw, const Con
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN_SMEM) != cudaSuccess) return -10;
   }
   const int tiles = ((cs.M + PG_BM - 1) / PG_BM) * ((cs.Cout + BN - 1) / BN) * cs.splitk;
-  const int resident = device_sm_count() * (L::DYN_SMEM <= 112 * 1024 && L::TMEM_COLS <= 256 ? 2 : 1);
+  const int resident = device_sm_count() * im2col_per_sm<BN, STAGES, KA>();
   const dim3 grid(tiles < resident ? tiles : resident);
   const uint32_t idesc = umma_idesc(PG_BM, BN, is_bf16 ? 1u : 0u, 1u);
   const cudaError_t err = launch(kern, grid, dim3(PG_THREADS), size_t(L::DYN_SMEM), stream, ma, mw, cs, e, idesc, status);
@@ -653,37 +662,33 @@ extern "C" int ronn_splitk_finalize(const float* ws, int S, const void* bias, co
                                     const void* gamma, const void* beta, void* y, long rows, int N, float eps,
                                     int act, int norm, int dtype, cudaStream_t stream);
 
-// x: NHWC [N, H, W, C]; w: [Cout, R, S, C] (K-major rows of R*S*C); out: NHWC [N, Ho, Wo, Cout];
-// out = act(conv(x, w) + bias + residual).  act 0 none, 1 ReLU.  C and Cout multiples of 8.  dtype 0 bf16, 1 fp16.
-// workspace (may be null): fp32 scratch of workspace_floats elements.  Layers whose output tiles cannot fill the GPU
-// but whose K loop is long (the deep 3x3 layers) run as K slices into fp32 panels there and are reduced, with
-// bias / residual / ReLU, by the split-K finalize kernel.
-extern "C" int ronn_conv2d(const void* x, const void* w, const void* bias, const void* residual, void* out, int N, int H,
-                           int W, int C, int Cout, int R, int S, int stride, int pad, int dil, int Ho, int Wo, int act,
-                           int dtype, float* workspace, long workspace_floats, uint32_t* status, cudaStream_t stream) {
-  if (N <= 0 || (C & 7) || (Cout & 7) || R <= 0 || S <= 0 || stride <= 0) return -2;
-  if (long(H) * W * C * N >= (1l << 31) || long(N) * Ho * Wo * Cout >= (1l << 31)) return -4;   // 32-bit offsets inside
-  ConvShape cs{N, H, W, C, Ho, Wo, Cout, R, S, stride, pad, dil, N * Ho * Wo, R * S * C / 8, 1, 0, pad};
-  const int Kg = R * S * C;
-  const int num_kb = (cs.chunks + 7) / 8;
-  const int m_tiles = (cs.M + 127) / 128;
-  // TMA im2col takes K blocks that lie in one filter tap (C a multiple of 64) or are four whole taps (C 16); corners and
-  // offsets that its descriptor cannot hold, and the other channel counts, go through the software gather.
-  CUtensorMap ma;
-  const bool tap16 = C == 16 && (R * S) % 4 == 0;
-  bool tma = (tap16 || (C & 63) == 0) && pad >= 0 && dil * (R - 1) < 256 && dil * (S - 1) < 256;
-  if (tma) tma = make_tmap_im2col(&ma, x, N, H, W, C, C, uint64_t(W) * C, uint64_t(H) * W * C, Ho, Wo, stride, pad, pad,
-                                  tap16 ? 16 : 64, PG_BM) == 0;
+// How a convolution runs: operand by TMA im2col or gathered, tile width, K slices.
+struct ConvPlan {
+  bool tma;
+  int bn, splitk;
+};
+
+// TMA im2col takes K blocks that lie in one filter tap (C a multiple of 64) or are four whole taps (C 16, tap16); corners and
+// offsets that its descriptor cannot hold, the other channel counts and narrow outputs go through the software gather.
+static bool conv_tap16(const ConvShape& cs) { return cs.C == 16 && (cs.R * cs.S) % 4 == 0; }
+static bool conv_by_tma(const ConvShape& cs) {
+  return (conv_tap16(cs) || (cs.C & 63) == 0) && cs.Cout >= 64 && cs.pad >= 0 && cs.dil * (cs.R - 1) < 256 && cs.dil * (cs.S - 1) < 256 &&
+         im2col_fits(cs.H, cs.W, cs.Ho, cs.Wo, cs.stride, cs.pad, cs.pad_w);
+}
+
+static ConvPlan conv_plan(const ConvShape& cs, bool tma, long workspace_floats) {
+  const int num_kb = (cs.chunks + 7) / 8, m_tiles = (cs.M + 127) / 128, Cout = cs.Cout, sms = device_sm_count();
+  const bool tap16 = conv_tap16(cs);
   int bn = Cout >= 128 ? 128 : (Cout >= 64 ? 64 : 32);
-  if (tma && bn < 64) tma = false;
   int splitk = 1;
   if (tma && !tap16) {
-    // Tile width and number of K slices: the cheapest by the microsecond model of the dense GEMM's forms (one main loop):
+    // Tile width and number of K slices: the cheapest by a model in microseconds like the dense GEMM's, with terms of its own
+    // (the operand comes by im2col loads, results of every form leave through the staging area, with bias and ReLU):
     // 256 and 128 wide with one CTA per SM, 64 wide with two; every wave pays its K blocks or, if longer, its epilogue.
     // K slices add the reduction kernel (3 us) and their fp32 panels, written and read at about 3 TB/s.  A model in K blocks
     // with a fixed price for the reduction sliced layers that one wave held anyway: 3x3 128 -> 256 / 2 at 28 x 28, batch 32:
-    // 25 us with three slices.
-    const int sms = device_sm_count();
+    // 25 us with three slices.  Over 3366 layers (batch 1 to 100, 7 to 113 pixels, 64 to 512 channels, 1x1 to 5x5) 1.8 times
+    // faster than the gather on average and never slower.
     float best = 1e30f;
     const int widths[3] = {256, 128, 64};
     for (int i = 0; i < 3; ++i) {
@@ -691,7 +696,7 @@ extern "C" int ronn_conv2d(const void* x, const void* w, const void* bias, const
       if (w > 64 && Cout < w) continue;
       const long tiles = long(m_tiles) * ((Cout + w - 1) / w);
       for (int sk = 1; sk <= 16; ++sk) {
-        if (sk > 1 && (workspace == nullptr || num_kb / sk < 4 || long(sk) * cs.M * Cout > workspace_floats)) break;
+        if (sk > 1 && (num_kb / sk < 4 || long(sk) * cs.M * Cout > workspace_floats)) break;
         const float kb = float((num_kb + sk - 1) / sk);
         const long n = tiles * sk;
         float t;
@@ -707,8 +712,8 @@ extern "C" int ronn_conv2d(const void* x, const void* w, const void* bias, const
     // layers with few output tiles comes from K slices, chosen by a small cost model in units of one K block: waves x (K
     // blocks per slice + fixed cost per tile) + the reduction pass.
     const int tiles = m_tiles * ((Cout + bn - 1) / bn);
-    const int resident = device_sm_count() * (bn >= 128 && !tap16 ? 1 : 2);
-    if (workspace != nullptr) {
+    const int resident = sms * (!tma ? (bn >= 128 ? 1 : 2) : (bn >= 128 ? im2col_per_sm<128, 3, 2>() : im2col_per_sm<64, 3, 1>()));
+    if (workspace_floats > 0) {
       int best = 1 << 30;
       for (int sk = 1; sk <= 8; ++sk) {
         if (sk > 1 && (num_kb / sk < 6 || long(sk) * cs.M * Cout > workspace_floats)) break;
@@ -717,9 +722,40 @@ extern "C" int ronn_conv2d(const void* x, const void* w, const void* bias, const
         if (cost < best) { best = cost; splitk = sk; }
       }
     } else if (!tma) {
-      while (bn > 32 && m_tiles * ((Cout + bn - 1) / bn) < 148) bn >>= 1;
+      while (bn > 32 && m_tiles * ((Cout + bn - 1) / bn) < sms) bn >>= 1;
     }
   }
+  return {tma, bn, splitk};
+}
+
+// The plan of a ronn_conv2d call: tile width | K slices << 12 | 1 << 20 where the operand comes by TMA im2col.
+extern "C" int ronn_conv2d_plan(int N, int H, int W, int C, int Cout, int R, int S, int stride, int pad, int dil, int Ho, int Wo,
+                                long workspace_floats) {
+  const ConvShape cs{N, H, W, C, Ho, Wo, Cout, R, S, stride, pad, dil, N * Ho * Wo, R * S * C / 8, 1, 0, pad};
+  const ConvPlan p = conv_plan(cs, conv_by_tma(cs), workspace_floats);
+  return p.bn | p.splitk << 12 | int(p.tma) << 20;
+}
+
+// x: NHWC [N, H, W, C]; w: [Cout, R, S, C] (K-major rows of R*S*C); out: NHWC [N, Ho, Wo, Cout];
+// out = act(conv(x, w) + bias + residual).  act 0 none, 1 ReLU.  C and Cout multiples of 8.  dtype 0 bf16, 1 fp16.
+// workspace (may be null): fp32 scratch of workspace_floats elements.  Layers whose output tiles cannot fill the GPU
+// but whose K loop is long (the deep 3x3 layers) run as K slices into fp32 panels there and are reduced, with
+// bias / residual / ReLU, by the split-K finalize kernel.
+extern "C" int ronn_conv2d(const void* x, const void* w, const void* bias, const void* residual, void* out, int N, int H,
+                           int W, int C, int Cout, int R, int S, int stride, int pad, int dil, int Ho, int Wo, int act,
+                           int dtype, float* workspace, long workspace_floats, uint32_t* status, cudaStream_t stream) {
+  if (N <= 0 || (C & 7) || (Cout & 7) || R <= 0 || S <= 0 || stride <= 0) return -2;
+  if (long(H) * W * C * N >= (1l << 31) || long(N) * Ho * Wo * Cout >= (1l << 31)) return -4;   // 32-bit offsets inside
+  ConvShape cs{N, H, W, C, Ho, Wo, Cout, R, S, stride, pad, dil, N * Ho * Wo, R * S * C / 8, 1, 0, pad};
+  const int Kg = R * S * C;
+  const int num_kb = (cs.chunks + 7) / 8;
+  const int m_tiles = (cs.M + 127) / 128;
+  const bool tap16 = conv_tap16(cs);
+  CUtensorMap ma;
+  const bool tma = conv_by_tma(cs) && make_tmap_im2col(&ma, x, N, H, W, C, C, uint64_t(W) * C, uint64_t(H) * W * C, Ho, Wo, stride, pad, pad,
+                                                       tap16 ? 16 : 64, PG_BM) == 0;
+  const ConvPlan plan = conv_plan(cs, tma, workspace != nullptr ? workspace_floats : 0);
+  const int bn = plan.bn, splitk = plan.splitk;
   cs.kb_per = (num_kb + splitk - 1) / splitk;
   cs.splitk = (num_kb + cs.kb_per - 1) / cs.kb_per;
   CUtensorMap mw;

@@ -40,6 +40,16 @@ inline EncodeIm2colFn encode_im2col_fn() {
   return fn;
 }
 
+// Whether the descriptor holds the window positions of an im2col tensor: they run from the lower corner to (size - 1 + upper
+// corner), both stored in 8 bits, in steps of up to 8.
+inline bool im2col_fits(int H, int W, int Ho, int Wo, int stride, int pad_h, int pad_w) {
+  const int lower[2] = {-pad_w, -pad_h};
+  const int upper[2] = {-pad_w + (Wo - 1) * stride - (W - 1), -pad_h + (Ho - 1) * stride - (H - 1)};
+  for (int i = 0; i < 2; ++i)
+    if (lower[i] < -128 || upper[i] < -128 || upper[i] > 127) return false;
+  return stride >= 1 && stride <= 8;
+}
+
 // NHWC tensor of 2-byte elements for im2col loads: a load starts at a filter window's top-left position (w, h of image n)
 // and takes `channels` channels at one filter tap of `pixels` consecutive output positions, in (w, h, n) order; the
 // windows are `stride` apart, Wo x Ho of them per image, the first at (-pad_w, -pad_h).  Positions outside the tensor, the
@@ -50,14 +60,11 @@ inline int make_tmap_im2col(CUtensorMap* map, const void* base, int N, int H, in
                             uint64_t n_stride, int Ho, int Wo, int stride, int pad_h, int pad_w, int channels, int pixels) {
   EncodeIm2colFn fn = encode_im2col_fn();
   if (!fn) return -1;
-  // the window positions run from the lower corner to (size - 1 + upper corner), both stored in 8 bits
+  if (!im2col_fits(H, W, Ho, Wo, stride, pad_h, pad_w) || (reinterpret_cast<uintptr_t>(base) & 15) || (w_stride & 7) ||
+      (h_stride & 7) || (n_stride & 7) || channels > C)
+    return -2;
   const int lower[2] = {-pad_w, -pad_h};
   const int upper[2] = {-pad_w + (Wo - 1) * stride - (W - 1), -pad_h + (Ho - 1) * stride - (H - 1)};
-  for (int i = 0; i < 2; ++i)
-    if (lower[i] < -128 || upper[i] < -128 || upper[i] > 127) return -2;
-  if (stride < 1 || stride > 8 || (reinterpret_cast<uintptr_t>(base) & 15) || (w_stride & 7) || (h_stride & 7) ||
-      (n_stride & 7) || channels > C)
-    return -2;
   cuuint64_t dims[4] = {cuuint64_t(C), cuuint64_t(W), cuuint64_t(H), cuuint64_t(N)};
   cuuint64_t strides[3] = {w_stride * 2, h_stride * 2, n_stride * 2};
   cuuint32_t estr[4] = {1, cuuint32_t(stride), cuuint32_t(stride), 1};

@@ -49,6 +49,7 @@ def declare(lib):
     sig("ronn_fmha", [V, L, L, I, I, I, V, V, V, V, L, I, I, I, I, I, I, F, I, V, V])
     sig("ronn_fmha_paged", [V, L, L, I, V, V, L, V, I, V, V, V, V, V, L, I, I, I, I, I, I, F, I, V, V])
     sig("ronn_conv2d", [V, V, V, V, V, I, I, I, I, I, I, I, I, I, I, I, I, I, I, V, L, V, V], optional=True)
+    sig("ronn_conv2d_plan", [I, I, I, I, I, I, I, I, I, I, I, I, L])
     sig("ronn_nchw_to_nhwc8", [V, V, I, I, I, I, I, V], optional=True)
     sig("ronn_stem_conv", [V, V, V, V, V, I, I, I, I, I, I, I, V, V])
     sig("ronn_nchw_to_s2d16", [V, V, I, I, I, I, I, V], optional=True)

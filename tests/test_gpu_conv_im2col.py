@@ -63,3 +63,30 @@ def test_stem_against_64_bits(shape, dtype):
     K.check_status()
     ref = F.relu(F.conv2d(x.double(), w.double(), b.double(), 2, 3)).permute(0, 2, 3, 1)
     assert y.shape == ref.shape and ((y.double() - ref).norm() / ref.norm()).item() < (2 ** -8 if dtype == torch.bfloat16 else 2 ** -11)
+
+
+# every form that a plan may take on a chip of 148 SMs; every value within its own bound, so that a lost or misplaced piece shows:
+# the rounding of the result (2^-11 for fp16) and K products summed in fp32 (K x 2^-23 of the sum of their magnitudes)
+@pytest.mark.parametrize("shape,want", [
+    ((40, 30, 29, 128, 256, 3, 3, 1, 1), (True, 256, 1)), ((40, 30, 29, 128, 128, 3, 3, 1, 1), (True, 128, 1)), ((33, 57, 55, 64, 72, 3, 3, 1, 1), (True, 64, 1)),
+    ((2, 20, 21, 64, 64, 1, 1, 1, 0), (True, 64, 1)), ((1, 7, 7, 512, 512, 3, 3, 1, 1), (True, None, None)), ((2, 57, 56, 16, 64, 4, 4, 1, 1), (True, 64, 1)),
+    ((2, 57, 56, 16, 136, 2, 2, 2, 0), (True, 128, 1)), ((1, 84, 84, 16, 128, 10, 10, 1, 2), (True, 128, 3)), ((2, 30, 31, 24, 136, 3, 3, 1, 1), (False, 128, None))])
+def test_every_plan_value_by_value(shape, want):
+    from ronn_b200 import _native
+    from ronn_b200.ops import kernels as K
+    from ronn_b200.providers.gpu_conv import conv2d_nhwc
+    N, H, W, C, Cout, R, S, stride, pad = shape
+    Ho, Wo = (H + 2 * pad - R) // stride + 1, (W + 2 * pad - S) // stride + 1
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        p = _native.cuda().ronn_conv2d_plan(N, H, W, C, Cout, R, S, stride, pad, 1, Ho, Wo, 1 << 22)
+        got = (bool(p >> 20), p & 0xfff, p >> 12 & 0xff)
+        assert all(w is None or w == v for w, v in zip(want, got)), got
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    x = torch.randn(N, H, W, C, generator=g, device="cuda").half()
+    w = (torch.randn(Cout, R, S, C, generator=g, device="cuda") / (R * S * C) ** 0.5).half()
+    b = torch.randn(Cout, generator=g, device="cuda").half()
+    y = conv2d_nhwc(x, w, b, None, stride, pad, 1, False)
+    K.check_status()
+    ref = _ref(x, w, b, None, stride, pad, 1, False)
+    bound = 2 ** -11 * ref.abs() + (R * S * C) * 2 ** -23 * _ref(x.abs(), w.abs(), b.abs(), None, stride, pad, 1, False) + 2 ** -24
+    assert y.shape == ref.shape and bool(((y.double() - ref).abs() <= bound).all())
