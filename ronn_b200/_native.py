@@ -134,7 +134,8 @@ def host():
 
 _NOT_LAUNCHERS = {"ronn_set_pdl", "ronn_set_rowwise_status", "ronn_no_alloc_scratch_floats", "ronn_no_alloc_strerror",
                   "ronn_gemm_fuse_state_ints", "ronn_gemm_fuse_flag_ints", "ronn_bitlinear_workspace_bytes",
-                  "ronn_bitlinear_slot_workspace_bytes", "ronn_gemm_form", "ronn_skinny_down_ok", "ronn_conv2d_plan"}
+                  "ronn_bitlinear_slot_workspace_bytes", "ronn_gemm_form", "ronn_gemm_ctas_per_sm", "ronn_skinny_down_ok",
+                  "ronn_conv2d_plan", "ronn_conv2d_ctas_per_sm"}
 
 
 class _Counted:

@@ -66,12 +66,14 @@ struct ConvSmem {
   static constexpr int TILE_BYTES = STAGES * STAGE_BYTES;
   static constexpr int DYN_SMEM = TILE_BYTES + (2 * STAGES + 4) * 8 + 16 + 1024;
   static constexpr uint32_t TMEM_COLS = 2 * BN <= 64 ? 64u : (2 * BN <= 128 ? 128u : (2 * BN <= 256 ? 256u : 512u));
+  // two CTAs per SM when shared memory (227 KB) and TMEM (512 columns) allow it; the launch bounds hold the registers to it
+  static constexpr int PER_SM = DYN_SMEM <= 110 * 1024 && TMEM_COLS <= 256 ? 2 : 1;
 };
 
 // Persistent: a CTA walks output tiles (tile = blockIdx.x, += gridDim.x); the smem ring and its barrier phases run
 // across tiles and the accumulator is double-buffered in TMEM, so the gather of tile j+1 overlaps the epilogue of j.
 template <int BN, class T, bool FAST>
-__global__ void __launch_bounds__(CONV_THREADS)
+__global__ void __launch_bounds__(CONV_THREADS, min_blocks(ConvSmem<BN>::PER_SM))
 conv_igemm_kernel(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_w, ConvShape cs, DenseEpilogue epi,
                   uint32_t idesc, uint32_t* status) {
   using L = ConvSmem<BN>;
@@ -263,7 +265,7 @@ conv_igemm_kernel(const T* __restrict__ x, const __grid_constant__ CUtensorMap m
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty[buf]);
-        epi.run<T>(row, 0, r0);
+        epi.run<T, L::PER_SM == 1>(row, 0, r0);
       } else {
         uint32_t r0[32], r1[32];
         tmem_ld_32x32(tacc, r0);
@@ -271,7 +273,7 @@ conv_igemm_kernel(const T* __restrict__ x, const __grid_constant__ CUtensorMap m
         for (int col = 0; col < BN; col += 64) {
           tmem_ld_wait();
           tmem_ld_32x32(tacc + uint32_t(col + 32), r1);
-          epi.run<T>(row, col, r0);
+          epi.run<T, L::PER_SM == 1>(row, col, r0);
           tmem_ld_wait();
           if (col + 64 < BN) {
             tmem_ld_32x32(tacc + uint32_t(col + 64), r0);
@@ -280,7 +282,7 @@ conv_igemm_kernel(const T* __restrict__ x, const __grid_constant__ CUtensorMap m
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[buf]);
           }
-          epi.run<T>(row, col + 32, r1);
+          epi.run<T, L::PER_SM == 1>(row, col + 32, r1);
         }
       }
     }
@@ -308,9 +310,7 @@ static int launch_conv_impl(const void* x, const CUtensorMap& mw, const ConvShap
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN_SMEM) != cudaSuccess) return -10;
   }
   const int sms = device_sm_count();
-  // two CTAs per SM when shared memory (227 KB) and TMEM (512 columns) allow it
-  const int per_sm = (L::DYN_SMEM <= 110 * 1024 && L::TMEM_COLS <= 256) ? 2 : 1;
-  const int resident = sms * per_sm;
+  const int resident = sms * L::PER_SM;
   const int tiles = ((cs.M + 127) / 128) * ((cs.Cout + BN - 1) / BN) * cs.splitk;
   dim3 grid(tiles < resident ? tiles : resident);
   const uint32_t idesc = umma_idesc(128, BN, is_bf16 ? 1u : 0u, 1u);
@@ -423,13 +423,6 @@ conv_im2col_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   gemm_persistent<BN, STAGES, 0, ConvProblem<BN, T, TAP16>, KA>(dyn_smem, prob, 64, idesc, status);
 }
 
-// CTAs of an im2col form that one SM holds: by its shared memory (two rings in 228 KB) and TMEM columns
-template <int BN, int STAGES, int KA>
-constexpr int im2col_per_sm() {
-  using L = PGemmSmem<BN, STAGES, true, KA>;
-  return L::DYN_SMEM <= 112 * 1024 && L::TMEM_COLS <= 256 ? 2 : 1;
-}
-
 template <int BN, int STAGES, int KA, class T, bool TAP16>
 static int launch_im2col(const CUtensorMap& ma, const CUtensorMap& mw, const ConvShape& cs, const DenseEpilogue& e, int is_bf16,
                          uint32_t* status, cudaStream_t stream) {
@@ -440,7 +433,7 @@ static int launch_im2col(const CUtensorMap& ma, const CUtensorMap& mw, const Con
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN_SMEM) != cudaSuccess) return -10;
   }
   const int tiles = ((cs.M + PG_BM - 1) / PG_BM) * ((cs.Cout + BN - 1) / BN) * cs.splitk;
-  const int resident = device_sm_count() * im2col_per_sm<BN, STAGES, KA>();
+  const int resident = device_sm_count() * L::PER_SM;
   const dim3 grid(tiles < resident ? tiles : resident);
   const uint32_t idesc = umma_idesc(PG_BM, BN, is_bf16 ? 1u : 0u, 1u);
   const cudaError_t err = launch(kern, grid, dim3(PG_THREADS), size_t(L::DYN_SMEM), stream, ma, mw, cs, e, idesc, status);
@@ -712,7 +705,7 @@ static ConvPlan conv_plan(const ConvShape& cs, bool tma, long workspace_floats) 
     // layers with few output tiles comes from K slices, chosen by a small cost model in units of one K block: waves x (K
     // blocks per slice + fixed cost per tile) + the reduction pass.
     const int tiles = m_tiles * ((Cout + bn - 1) / bn);
-    const int resident = sms * (!tma ? (bn >= 128 ? 1 : 2) : (bn >= 128 ? im2col_per_sm<128, 3, 2>() : im2col_per_sm<64, 3, 1>()));
+    const int resident = sms * (!tma ? (bn >= 128 ? ConvSmem<128>::PER_SM : ConvSmem<64>::PER_SM) : (bn >= 128 ? PGemmSmem<128, 3, true, 2>::PER_SM : PGemmSmem<64, 3, true, 1>::PER_SM));
     if (workspace_floats > 0) {
       int best = 1 << 30;
       for (int sk = 1; sk <= 8; ++sk) {
@@ -734,6 +727,21 @@ extern "C" int ronn_conv2d_plan(int N, int H, int W, int C, int Cout, int R, int
   const ConvShape cs{N, H, W, C, Ho, Wo, Cout, R, S, stride, pad, dil, N * Ho * Wo, R * S * C / 8, 1, 0, pad};
   const ConvPlan p = conv_plan(cs, conv_by_tma(cs), workspace_floats);
   return p.bn | p.splitk << 12 | int(p.tma) << 20;
+}
+
+// CTAs of a convolution form that one SM of the current device holds, or a negative error; its grid and its plan count PER_SM.
+template <int BN, class T>
+static int gather_resident() { return resident_ctas(conv_igemm_kernel<BN, T, false>, CONV_THREADS, ConvSmem<BN>::DYN_SMEM); }
+extern "C" int ronn_conv2d_ctas_per_sm(int tma, int bn, int dtype) {
+  if (tma && bn == 64) return resident_ctas(conv_im2col_kernel<64, 3, 1, __half, false>, PG_THREADS, PGemmSmem<64, 3, true, 1>::DYN_SMEM);
+  if (tma && bn == 128) return resident_ctas(conv_im2col_kernel<128, 3, 2, __half, false>, PG_THREADS, PGemmSmem<128, 3, true, 2>::DYN_SMEM);
+  if (tma) return -3;
+  switch (bn) {
+    case 32: return dtype == 0 ? gather_resident<32, __nv_bfloat16>() : gather_resident<32, __half>();
+    case 64: return dtype == 0 ? gather_resident<64, __nv_bfloat16>() : gather_resident<64, __half>();
+    case 128: return dtype == 0 ? gather_resident<128, __nv_bfloat16>() : gather_resident<128, __half>();
+    default: return -3;
+  }
 }
 
 // x: NHWC [N, H, W, C]; w: [Cout, R, S, C] (K-major rows of R*S*C); out: NHWC [N, Ho, Wo, Cout];

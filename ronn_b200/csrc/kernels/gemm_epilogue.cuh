@@ -4,6 +4,24 @@
 
 namespace ronn {
 
+// Second launch bound of a kernel that runs `per_sm` CTAs per SM: 0 (no bound) for one.
+constexpr int min_blocks(int per_sm) { return per_sm > 1 ? per_sm : 0; }
+
+// CTAs of a kernel that one SM of the current device holds by registers (whole groups of 8 per thread) and shared memory, or a
+// negative error.  cudaOccupancyMaxActiveBlocksPerMultiprocessor answers 1 for every kernel that uses TMEM.
+template <class Kernel>
+int resident_ctas(Kernel kern, int threads, int dyn_smem) {
+  cudaFuncAttributes a;
+  int dev = 0, regs = 0, smem = 0, reserved = 0;
+  if (cudaFuncGetAttributes(&a, kern) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&regs, cudaDevAttrMaxRegistersPerMultiprocessor, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess)
+    return -12;
+  const int by_regs = regs / ((a.numRegs + 7) / 8 * 8 * threads), by_smem = smem / (dyn_smem + int(a.sharedSizeBytes) + reserved);
+  return by_regs < by_smem ? by_regs : by_smem;
+}
+
 struct DenseEpilogue {
   void* C;
   const void* bias;        // [N] in the operand dtype, or null
@@ -17,7 +35,11 @@ struct DenseEpilogue {
   // `stage` (optional): 32 x 80 bytes of shared memory owned by the calling warp.  With it, and when the whole warp
   // calls with the same `col`, 16-bit results leave as 64 contiguous bytes per row from 4 lanes (8 rows per store
   // instruction) instead of 32 rows of 16 bytes, which halves the number of write transactions and fills every sector.
-  template <class T>
+  // EARLY: the residual row is fetched before the bias and the activation, which hides its latency and costs 16 registers.  Forms
+  // that run two CTAs per SM cannot pay them (102 registers per thread) and hide it behind the other CTA: with the early fetch the
+  // shallow 128-wide GEMM and the 64-wide gather convolution went from 96 to 132 registers and ran one CTA per SM (norm + 1 x 32000
+  // x 64: 6.9 -> 9.9 us).
+  template <class T, bool EARLY = true>
   __device__ __forceinline__ void run(int row, int col, uint32_t (&r)[32], uint8_t* stage = nullptr) const {
     const int gm = m0 + row;
     const int gn = n0 + col;
@@ -37,19 +59,19 @@ struct DenseEpilogue {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
     const bool full = (gn + 32 <= N) && ((ldc & 7) == 0);
-    // the residual row is fetched first: its latency passes under the bias and the activation
-    Vec8 rp[4];
-    if (residual && full) {
+    Vec8 rp[EARLY ? 4 : 1];
+    if (EARLY && residual && full) {
       const T* res = reinterpret_cast<const T*>(residual) + size_t(gm) * ldc + gn;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) rp[j] = *reinterpret_cast<const Vec8*>(res + j * 8);
+      for (int j = 0; j < (EARLY ? 4 : 0); ++j) rp[j] = *reinterpret_cast<const Vec8*>(res + j * 8);
     }
     auto add_residual = [&]() {
       if (full) {
+        const T* res = reinterpret_cast<const T*>(residual) + size_t(gm) * ldc + gn;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           float f[8];
-          unpack8<T>(rp[j], f);
+          unpack8<T>(EARLY ? rp[EARLY ? j : 0] : *reinterpret_cast<const Vec8*>(res + j * 8), f);
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[j * 8 + i] += f[i];
         }

@@ -20,7 +20,7 @@ namespace ronn {
 
 // Tile list of a dense (optionally split-K) GEMM for the persistent mainloop.  Tiles are numbered with the
 // M index fastest so that CTAs running side by side share the same weight tile in L2.
-template <int BN, class T>
+template <int BN, class T, bool EARLY>
 struct DenseProblem {
   static constexpr bool kForceStage = false;
   const CUtensorMap* map_a;
@@ -49,16 +49,17 @@ struct DenseProblem {
     ep.n0 = n0;
     if (splitk > 1)     // raw fp32 partial sums go to slice z of the workspace
       ep.C = reinterpret_cast<float*>(e.C) + size_t(t / (m_tiles * n_tiles)) * size_t(e.M) * size_t(e.ldc);
-    ep.run<T>(row, col, r, stage);
+    ep.run<T, EARLY>(row, col, r, stage);
   }
 };
 
 template <int BN, int STAGES, class T, int KA>
-__global__ void __launch_bounds__(PG_THREADS)
+__global__ void __launch_bounds__(PG_THREADS, min_blocks(PGemmSmem<BN, STAGES, false, KA>::PER_SM))
 gemm_dense_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   DenseEpilogue epi, int K, int splitk, uint32_t idesc, uint32_t* status) {
   extern __shared__ uint8_t dyn_smem[];
-  DenseProblem<BN, T> prob;
+  using Problem = DenseProblem<BN, T, PGemmSmem<BN, STAGES, false, KA>::PER_SM == 1>;
+  Problem prob;
   prob.map_a = &map_a;
   prob.map_b = &map_b;
   prob.e = epi;
@@ -67,7 +68,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   prob.num_kb = (K + 63) / 64;
   prob.splitk = splitk;
   prob.kb_per = (prob.num_kb + splitk - 1) / splitk;
-  gemm_persistent<BN, STAGES, 0, DenseProblem<BN, T>, KA>(dyn_smem, prob, 64, idesc, status);
+  gemm_persistent<BN, STAGES, 0, Problem, KA>(dyn_smem, prob, 64, idesc, status);
 }
 
 static int sm_count() { return device_sm_count(); }
@@ -144,7 +145,7 @@ static int launch_dense(const CUtensorMap& ma, const CUtensorMap& mb, DenseEpilo
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN_SMEM) != cudaSuccess) return -10;
   }
   const int tiles = ((N + BN - 1) / BN) * ((M + PG_BM - 1) / PG_BM) * splitk;
-  const int resident = sm_count() * (L::DYN_SMEM <= 112 * 1024 && L::TMEM_COLS <= 256 ? 2 : 1);
+  const int resident = sm_count() * L::PER_SM;
   dim3 grid(tiles < resident ? tiles : resident);
   uint32_t idesc = umma_idesc(PG_BM, BN, is_bf16 ? 1u : 0u, 1u);
   cudaError_t err = launch(kern, grid, dim3(PG_THREADS), size_t(L::DYN_SMEM), stream, ma, mb, epi, K, splitk, idesc, status);
@@ -182,6 +183,8 @@ constexpr int FORM_SKINNY = 0x8000, FORM_CTA_PAIR = 0x4000, FORM_SHALLOW = 0x200
 // What it has to weigh, us: 1024 x 64 x 1024 fp32 8.1 at 32 wide, 9.7 at 64 shallow; 1024 x 768 x 2048 12.3 at 64 deep, 14.6
 // shallow; 8192 x 2304 x 64 residual 23.8 on pairs, 34.4 at 64; 8192 x 3072 x 768 GELU 43.4 / 55.0 / 52.7 on pairs / 256 / 128;
 // 4662 x 50257 x 768 (odd rows) 412 / 627 on pairs / 256.
+// The shallow 128-wide entry was measured while its 132 registers let one CTA run per SM where two are launched; with two it
+// costs less, so the entry keeps the form from being chosen rather than choosing it wrongly.
 struct FormCost {
   int form;
   float start_one, start_more, block_one, block_more, epilogue, gelu, residual, fp32, ragged, gap, drain;
@@ -266,6 +269,25 @@ extern "C" int ronn_gemm_skinny(const void* A, const void* W, void* C, const voi
 // The form that ronn_gemm runs for these arguments (see gemm_form).
 extern "C" int ronn_gemm_form(int M, int N, int K, int act, int residual, int out_fp32, long ldc, int bn) {
   return gemm_form(M, N, K, act, residual != 0, out_fp32 != 0, ldc, bn);
+}
+
+// CTAs of a tile form (its code as ronn_gemm_form gives it) that one SM of the current device holds, or a negative error.
+// The launch sizes its grid for PER_SM of them.
+extern "C" int ronn_gemm_ctas_per_sm(int form, int dtype) {
+#define RONN_RESIDENT(BN_, ST_, KA_)                                                                                 \
+  return dtype == 0 ? resident_ctas(gemm_dense_kernel<BN_, ST_, __nv_bfloat16, KA_>, PG_THREADS, PGemmSmem<BN_, ST_, false, KA_>::DYN_SMEM) \
+                    : resident_ctas(gemm_dense_kernel<BN_, ST_, __half, KA_>, PG_THREADS, PGemmSmem<BN_, ST_, false, KA_>::DYN_SMEM)
+  switch (form) {
+    case 32 | FORM_SHALLOW: RONN_RESIDENT(32, 5, 1);
+    case 64 | FORM_SHALLOW: RONN_RESIDENT(64, 4, 1);
+    case 128 | FORM_SHALLOW: RONN_RESIDENT(128, 3, 1);
+    case 32 | FORM_DEEP: RONN_RESIDENT(32, 5, 2);
+    case 64 | FORM_DEEP: RONN_RESIDENT(64, 4, 2);
+    case 128 | FORM_DEEP: RONN_RESIDENT(128, 3, 2);
+    case 256: RONN_RESIDENT(256, 4, 1);
+    default: return -3;
+  }
+#undef RONN_RESIDENT
 }
 
 // dtype: 0 = bf16, 1 = fp16.  act: 0 none, 1 relu, 2 gelu.  bn: 0 = auto, else 32|64|128|256, or 256 | 0x4000 for CTA

@@ -59,6 +59,8 @@ struct PGemmSmem {
   static constexpr int TOTAL = TILE_BYTES + NUM_BARS * 8 + 16 + OUT_STAGE_BYTES;
   static constexpr int DYN_SMEM = TOTAL + 1024;            // slack for manual 1024-byte alignment
   static constexpr uint32_t TMEM_COLS = (2 * BN <= 32) ? 32u : (2 * BN <= 64 ? 64u : (2 * BN <= 128 ? 128u : (2 * BN <= 256 ? 256u : 512u)));
+  // CTAs of this form that one SM holds by shared memory and TMEM; the launch bounds of its kernel hold the registers to it
+  static constexpr int PER_SM = DYN_SMEM <= 112 * 1024 && TMEM_COLS <= 256 ? 2 : 1;
 };
 
 // KIND: 0 = f16/bf16 operands, 1 = int8 operands.  k_elems: K elements per 128-byte smem row (64 or 128).

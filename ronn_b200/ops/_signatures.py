@@ -17,6 +17,7 @@ def declare(lib):
 
     sig("ronn_gemm", [V, V, V, V, V, I, I, I, I, I, I, I, I, I, I, V, V])
     sig("ronn_gemm_form", [I, I, I, I, I, I, L, I])
+    sig("ronn_gemm_ctas_per_sm", [I, I])
     sig("ronn_skinny_down_ok", [I, I, I])
     sig("ronn_gemm_skinny", [V, V, V, V, V, V, V, F, I, I, I, I, L, L, L, I, I, I, V])
     sig("ronn_gemm_splitk", [V, V, V, I, I, I, I, I, I, I, I, V, V, V])
@@ -49,6 +50,7 @@ def declare(lib):
     sig("ronn_fmha", [V, L, L, I, I, I, V, V, V, V, L, I, I, I, I, I, I, F, I, V, V])
     sig("ronn_fmha_paged", [V, L, L, I, V, V, L, V, I, V, V, V, V, V, L, I, I, I, I, I, I, F, I, V, V])
     sig("ronn_conv2d", [V, V, V, V, V, I, I, I, I, I, I, I, I, I, I, I, I, I, I, V, L, V, V], optional=True)
+    sig("ronn_conv2d_ctas_per_sm", [I, I, I])
     sig("ronn_conv2d_plan", [I, I, I, I, I, I, I, I, I, I, I, I, L])
     sig("ronn_nchw_to_nhwc8", [V, V, I, I, I, I, I, V], optional=True)
     sig("ronn_stem_conv", [V, V, V, V, V, I, I, I, I, I, I, I, V, V])

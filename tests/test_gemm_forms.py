@@ -137,3 +137,16 @@ def test_calls_between_the_rows_of_a_tile():
             for fp32 in (False, True):
                 f = form(M, N, 8, fp32=fp32, ldc=N)
                 assert f in known and not (fp32 and f & PAIR), (M, N, fp32, hex(f))
+
+
+# the grids of these forms, and the rules that choose them, count two CTAs per SM: registers have to fit as well
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_two_ctas_fit_an_sm(dtype):
+    lib = _native.cuda()
+    for bn in (32, 64, 128):
+        assert lib.ronn_gemm_ctas_per_sm(bn | SHALLOW, dtype) >= 2 and lib.ronn_gemm_ctas_per_sm(bn | DEEP, dtype) == 1
+    assert lib.ronn_gemm_ctas_per_sm(256, dtype) == 1
+    for bn, per_sm in ((32, 2), (64, 2), (128, 1)):
+        assert lib.ronn_conv2d_ctas_per_sm(0, bn, dtype) >= per_sm
+    assert lib.ronn_conv2d_ctas_per_sm(1, 64, dtype) == 2 and lib.ronn_conv2d_ctas_per_sm(1, 128, dtype) == 1
