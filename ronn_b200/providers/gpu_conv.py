@@ -71,15 +71,18 @@ def stem_conv_s2d(x_nchw, w2, bias, relu):
     into its 2x2 space-to-depth NHWC form, the implicit-GEMM kernel then runs a 4x4 stride-1 convolution with K = 256."""
     N, C, H, W = x_nchw.shape
     Cout, dt = w2.shape[0], 0 if x_nchw.dtype == torch.bfloat16 else 1
-    out = torch.empty((N, H // 2, W // 2, Cout), dtype=x_nchw.dtype, device=x_nchw.device)
-    scratch = torch.empty(N * (H // 2) * (W // 2 + 3) * 16, dtype=x_nchw.dtype, device=x_nchw.device)
-    rc = _native.cuda().ronn_stem_conv(x_nchw.data_ptr(), w2.data_ptr(), None if bias is None else bias.data_ptr(), out.data_ptr(),
-                                       scratch.data_ptr(), N, C, H, W, Cout, 1 if relu else 0, dt,
-                                       K.status_word(x_nchw.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
-    if rc == 0:
-        return out
-    if rc != -2:                                    # -2: a size the one-call form does not take, nothing was launched
-        raise K.KernelError(f"stem_conv failed with code {rc}")
+    padded = N * (H // 2) * (W // 2 + 3) * 16
+    if Cout >= 64 and Cout % 8 == 0 and padded < 1 << 31:          # what the one-call form may take: no memory for the others
+        out = torch.empty((N, H // 2, W // 2, Cout), dtype=x_nchw.dtype, device=x_nchw.device)
+        scratch = torch.empty(padded, dtype=x_nchw.dtype, device=x_nchw.device)
+        rc = _native.cuda().ronn_stem_conv(x_nchw.data_ptr(), w2.data_ptr(), None if bias is None else bias.data_ptr(), out.data_ptr(),
+                                           scratch.data_ptr(), N, C, H, W, Cout, 1 if relu else 0, dt,
+                                           K.status_word(x_nchw.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+        if rc == 0:
+            return out
+        if rc != -2:                                # -2: refused (larger than its 32-bit offsets hold), nothing was launched
+            raise K.KernelError(f"stem_conv failed with code {rc}")
+        del out, scratch
     x2 = torch.empty((N, H // 2, W // 2, 16), dtype=x_nchw.dtype, device=x_nchw.device)
     rc = _native.cuda().ronn_nchw_to_s2d16(x_nchw.data_ptr(), x2.data_ptr(), N, C, H, W,
                                            0 if x_nchw.dtype == torch.bfloat16 else 1,

@@ -35,3 +35,23 @@ def test_slices_fit_the_workspace():
         for c in (64, 128, 256, 512):
             tma, bn, slices = plan(n, 14, 14, c, c, 3, 3, 1, 1)
             assert slices == 1 or slices * n * 196 * c <= WORKSPACE
+
+
+# the image network's first convolution: sizes that the one-call form never takes ask it for nothing and allocate nothing for it
+@pytest.mark.parametrize("cout,one_call", [(64, True), (72, True), (40, False), (68, False)])
+def test_stem_allocates_for_the_form_that_runs(cout, one_call, monkeypatch):
+    from types import SimpleNamespace
+
+    import torch
+
+    from ronn_b200.providers import gpu_conv as G
+    calls, sizes, empty = [], [], torch.empty
+    lib = SimpleNamespace(ronn_stem_conv=lambda *a: calls.append("stem") or 0, ronn_nchw_to_s2d16=lambda *a: calls.append("s2d") or 0)
+    monkeypatch.setattr(G._native, "cuda", lambda: lib)
+    monkeypatch.setattr(G.K, "status_word", lambda device: torch.zeros(4, dtype=torch.int32))
+    monkeypatch.setattr(G.torch.cuda, "current_stream", lambda: SimpleNamespace(cuda_stream=0))
+    monkeypatch.setattr(G.torch, "empty", lambda shape, **kw: sizes.append(shape) or empty(shape, **kw))
+    monkeypatch.setattr(G, "conv2d_nhwc", lambda *a, **kw: calls.append("conv"))
+    G.stem_conv_s2d(torch.zeros(1, 3, 8, 12, dtype=torch.float16), torch.zeros(cout, 4, 4, 16, dtype=torch.float16), None, True)
+    assert calls == (["stem"] if one_call else ["s2d", "conv"])
+    assert sizes == ([(1, 4, 6, cout), 4 * 9 * 16] if one_call else [(1, 4, 6, 16)])
