@@ -317,7 +317,8 @@ static int dispatch_skinny(const SkinnyArgs& a, cudaStream_t stream) {
 //
 // Up to 16 rows it reads the weights once and wins (N 10 to 50257, K 64 to 8192), but for 9 to 16 rows against matrices of
 // 64 Mi values and more that the other kernel holds in one wave: 12 x 8192 x 8192 40 / 37 us, 16 x 16384 x 4096 37 / 28.
-// What it still loses there: 8 x 16384 x 8192 63 / 51, 16 x 16384 x 1536 19 / 16, 16 x 8192 x 4096 and 5120 by 8 %.
+// What it still loses there: 16 x 32000 x 4096 69 / 51, 8 x 16384 x 8192 63 / 52, 12 x 32000 x 1536 35 / 29, 16 x 16384 x 1536 20 /
+// 17, 1 x 50257 x 1536 51 / 44, 1 x 50257 x 256 11.9 / 10.5.
 // K of up to 128 gives one or two of the 8 warps weights to read: the vocabulary of a very narrow model, behind its norm kernel,
 // is left to tcgen05 (1 to 8 x 50257 x 64 11.2 / 8.7 with the norm, x 32000 x 128 8.8 / 8.1; x 16384 x 64 stays, 5.6 / 7.0).
 //
@@ -326,7 +327,7 @@ static int dispatch_skinny(const SkinnyArgs& a, cudaStream_t stream) {
 //   skinny   1.1 + waves of CTAs x (0.6 + 0.24 per 8 weight rows of a CTA) + 0.46 per million weights and slice
 //   tcgen05  3.15 + 0.23 per K block + 0.23 per million weights, and when the tiles are more than the SMs
 //            5.6 per further wave of two tiles per SM + 0.36 per K block and wave
-// Where it names the skinny kernel the other is at most 8 % faster; where it names the other, 15 sizes of N 3072 and more and
+// Where it names the skinny kernel the other is at most 9 % faster; where it names the other, 15 sizes of N 3072 and more and
 // K 512 to 1536 would be 5 to 24 % faster here (40 x 3072 x 1024 7.8 / 9.2, 17 x 50257 x 1024 35 / 43).  By weights and slices alone (a line at 12 Mi values) short K went to the wrong side: 96 x 16384 x 64 19.7 / 5.2 us, 64 x 3072
 // x 1024 10.1 / 7.5, and long K stayed on it: 64 x 1024 x 4096 11.9 / 18.7.
 //   us, skinny / tcgen05   N 3072 K 1024   N 1024 K 1024   N 768 K 768   N 1024 K 4096   N 8192 K 256
